@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(NT) k_coef_solve2d(Params<T> P, const T *coef,
         double *part = partials + (size_t)(pass & 1) * KS * G;
         block_partials<KS, KS, NT>(&wred[0][0], part, G);
         if (!grid_sync(bar, G, epoch)) { failed = true; break; }
-        reduce_partials<KS, NT>(part, G, tot);
+        reduce_partials<NT>(part, KS, G, tot);
         // the rule of finish_sweeps, evaluated identically in every CTA
         bool stop_now = false;
         for (int s = 0; s < ns; ++s) {

@@ -158,59 +158,89 @@ void Engine<T>::enq_fused_rc()
 namespace ifc {
 
 // ---- the persistent single-launch 2D solve (ifc_persist2d.cuh) ----
-// launch = false: set the kernel's shared-memory limit and return in *capacity
-// the CTAs that can be co-resident.  launch = true: launch it on e.persist_grid
-// CTAs (e.persist_mt: several tiles per CTA).
-template <typename T, int KS, bool MT>
+// Region shapes: rows per lane and warps (a region is 64 x R*NW cells).  The
+// shape with the least estimated time per pass is taken: rounds of tiles per
+// CTA times the shape's cost of a pass (relative time of a half sweep).  Small
+// grids leave SMs idle, so the smallest region with the shortest half sweep
+// wins as long as its tiles fit one round (64x64 cavity: 69 ms to convergence
+// with 24 rows, 77 with 32; FP64 500x36: 113 against 148 us per iteration);
+// the larger regions waste less on halos and win once they save a round
+// (1024x256: 112 us with 64 rows; 32 rows would take 4 rounds).  FP64 has half
+// the registers per cell: 64 rows do not fit, 36 rows (500x190 in one round)
+// do.
+struct RegionShape {
+    int R, NW;
+    double cost;
+};
+template <typename T>
+struct RegionShapes;
+template <>
+struct RegionShapes<float> {
+    static constexpr int n = 3;
+    static constexpr RegionShape s[n] = {{2, 12, 0.85}, {2, 16, 1.0}, {4, 16, 1.6}};
+};
+template <>
+struct RegionShapes<double> {
+    static constexpr int n = 3;
+    static constexpr RegionShape s[n] = {{2, 12, 0.8}, {2, 16, 1.0}, {2, 18, 1.1}};
+};
+
+template <typename T, int I>
+using ShapeTile = RTile<T, RegionShapes<T>::s[I].R, RegionShapes<T>::s[I].NW>;
+
+// Dynamic shared memory of k_simple2d: exchange rows of two fields, then the
+// per-thread sums of a pass or (Rhie-Chow) the faces of a tile.
+template <typename RT, typename T>
+static size_t persist_smem(int ks)
+{
+    const size_t sums = (size_t)(2 * ks > 7 ? 2 * ks : 7) * RT::NT * sizeof(double);
+    const size_t faces = ((size_t)(RT::W + 1) * RT::HR + (size_t)RT::W * (RT::HR + 1)) * sizeof(T);
+    return (size_t)RT::END * sizeof(T) + (sums > faces ? sums : faces);
+}
+
+// launch = false: set the kernel's shared-memory limit (one setting per process,
+// so the device's maximum) and return in *capacity the CTAs that can be
+// co-resident.  launch = true: launch it on e.persist_grid CTAs.
+template <typename T, int I>
 static int persist_kernel(Engine<T> &e, bool launch, int *capacity)
 {
-    using S = TileShape2D<T>;
-    using R = Region<S::TX, S::TY, 2 * KS>;
-    const size_t smem = (size_t)3 * R::NR * sizeof(T);
-    auto kern = k_simple2d<T, S::TX, S::TY, KS, S::NT, MT>;
+    using RT = ShapeTile<T, I>;
+    auto kern = k_simple2d<T, RT::R, RT::NW>;
+    const size_t smem = persist_smem<RT, T>(e.persist_args.ks);
     if (!launch) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        int dev = 0, optin = 0;
+        cudaFuncAttributes fa;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+            cudaFuncGetAttributes(&fa, kern) != cudaSuccess)
+            return IFC_CUDA_ERROR;
+        const int dyn_max = optin - (int)fa.sharedSizeBytes;
+        if ((long long)smem > dyn_max) return IFC_UNSUPPORTED;  // deep passes of the largest region
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn_max) != cudaSuccess)
             return IFC_CUDA_ERROR;
         int per_sm = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, S::NT, smem) != cudaSuccess)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, RT::NT, smem) != cudaSuccess)
             return IFC_CUDA_ERROR;
-        *capacity = per_sm * e.nsm;
+        *capacity = (per_sm < 2 ? per_sm : 2) * e.nsm;
         return IFC_OK;
     }
-    PersistArgs pa;
-    pa.n_iter[0] = e.cfg.n_iter_u;
-    pa.n_iter[1] = e.cfg.n_iter_v;
-    pa.n_iter[2] = 0;
-    pa.n_iter[3] = e.cfg.n_iter_p;
-    pa.pin = e.pin ? 1 : 0;
+    PersistArgs &pa = e.persist_args;
     const char *stall = std::getenv("IFC_TEST_STALL_BARRIER");
     pa.stall_test = (stall && stall[0] == '1') ? 1 : 0;
     void *args[] = {&e.P, &e.f, &e.ctl, &e.partials, &e.barrier, &pa};
-    return cudaLaunchCooperativeKernel((const void *)kern, dim3(e.persist_grid), dim3(S::NT), args, smem, e.stream) ==
+    return cudaLaunchCooperativeKernel((const void *)kern, dim3(e.persist_grid), dim3(RT::NT), args, smem, e.stream) ==
                    cudaSuccess
                ? IFC_OK
                : IFC_CUDA_ERROR;
 }
 
-template <typename T, bool MT>
-static int persist_dispatch_t(Engine<T> &e, int ks, bool launch, int *capacity)
-{
-    switch (ks) {
-    case 2: return persist_kernel<T, 2, MT>(e, launch, capacity);
-    case 3: return persist_kernel<T, 3, MT>(e, launch, capacity);
-    case 4: return persist_kernel<T, 4, MT>(e, launch, capacity);
-    case 5: return persist_kernel<T, 5, MT>(e, launch, capacity);
-    case 6: return persist_kernel<T, 6, MT>(e, launch, capacity);
-    case 8: return persist_kernel<T, 8, MT>(e, launch, capacity);
-    default: return persist_kernel<T, 10, MT>(e, launch, capacity);
-    }
-}
-
 template <typename T>
-static int persist_dispatch(Engine<T> &e, int ks, bool launch, int *capacity, bool mt)
+static int persist_dispatch(Engine<T> &e, int shape, bool launch, int *capacity)
 {
-    return mt ? persist_dispatch_t<T, true>(e, ks, launch, capacity)
-              : persist_dispatch_t<T, false>(e, ks, launch, capacity);
+    constexpr int n = RegionShapes<T>::n;
+    if (shape == n - 1) return persist_kernel<T, n - 1>(e, launch, capacity);
+    if (shape == n - 2) return persist_kernel<T, n - 2>(e, launch, capacity);
+    return persist_kernel<T, 0>(e, launch, capacity);
 }
 
 static inline int persist_ks(int want)
@@ -221,15 +251,14 @@ static inline int persist_ks(int want)
 }
 
 // The whole 2D loop as one cooperative launch: one tile per CTA when all tiles'
-// CTAs can be co-resident, otherwise (MT) every CTA visits ceil(tiles / CTAs)
-// tiles in turn, on the fewest CTAs that give that count (so every CTA has the
-// same number of tiles but the last ones).  IFC_PERSIST_OFF=1 keeps the multi-kernel graph; IFC_PERSIST_MAX_CTAS caps the CTAs
-// (used by the tests to run the multi-tile form on small grids).
+// CTAs can be co-resident, otherwise every CTA visits ceil(tiles / CTAs) tiles
+// in turn, on the fewest CTAs that give that count.  IFC_PERSIST_OFF=1 keeps
+// the multi-kernel graph; IFC_PERSIST_MAX_CTAS caps the CTAs (used by the tests
+// to run several tiles per CTA on small grids).
 template <typename T>
 int Engine<T>::prepare_persist()
 {
     persist = false;
-    persist_mt = false;
     if (dim != 2 || !fused || cfg.linear_solver != IFC_GAUSS_SEIDEL) return IFC_OK;
     // the residual rule needs the residual pass of the graph form
     if (P.g.criterion == 2) return IFC_OK;
@@ -238,30 +267,40 @@ int Engine<T>::prepare_persist()
     int coop = 0, dev = 0;
     cudaGetDevice(&dev);
     if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop) return IFC_OK;
-    const int ks = persist_ks(spp_persist);
-    int capacity = 0, capacity_mt = 0;
-    if (persist_dispatch<T>(*this, ks, false, &capacity, false) != IFC_OK ||
-        persist_dispatch<T>(*this, ks, false, &capacity_mt, true) != IFC_OK) {
-        cudaGetLastError();
-        return IFC_OK;
-    }
-    if (const char *cap = std::getenv("IFC_PERSIST_MAX_CTAS")) {
-        const int c = std::atoi(cap);
-        if (c > 0) {
-            capacity = capacity < c ? capacity : c;
-            capacity_mt = capacity_mt < c ? capacity_mt : c;
+    PersistArgs &pa = persist_args;
+    pa.n_iter[0] = cfg.n_iter_u;
+    pa.n_iter[1] = cfg.n_iter_v;
+    pa.n_iter[2] = 0;
+    pa.n_iter[3] = cfg.n_iter_p;
+    pa.pin = pin ? 1 : 0;
+    pa.ks = persist_ks(spp_persist);
+    pa.stall_test = 0;
+    int cap_env = 0;
+    if (const char *cap = std::getenv("IFC_PERSIST_MAX_CTAS")) cap_env = std::atoi(cap);
+    double best = 0.0;
+    for (int s = 0; s < RegionShapes<T>::n; ++s) {
+        const RegionShape &sh = RegionShapes<T>::s[s];
+        TileGrid tg;
+        tg.H = 2 * pa.ks;
+        if (!split_axis(P.g.nx, 64, tg.H, &tg.kx, &tg.Ix) || !split_axis(P.g.ny, sh.R * sh.NW, tg.H, &tg.ky, &tg.Iy))
+            continue;
+        int capacity = 0;
+        if (persist_dispatch<T>(*this, s, false, &capacity) != IFC_OK) {
+            cudaGetLastError();
+            continue;
         }
-    }
-    using S = TileShape2D<T>;
-    const int tiles = ((P.g.nx + S::TX - 1) / S::TX) * ((P.g.ny + S::TY - 1) / S::TY);
-    if (tiles <= capacity) {
+        if (cap_env > 0 && capacity > cap_env) capacity = cap_env;
+        if (capacity < 1) continue;
+        const long long tiles = (long long)tg.kx * tg.ky;
+        const long long per = (tiles + capacity - 1) / capacity;
+        // (a single tile runs without grid barriers)
+        const double cost = (double)per * sh.cost - (tiles == 1 ? 0.3 : 0.0);
+        if (persist && cost >= best) continue;
+        best = cost;
         persist = true;
-        persist_grid = tiles;
-    } else if (capacity_mt > 0) {
-        const int per = (tiles + capacity_mt - 1) / capacity_mt;
-        persist = true;
-        persist_mt = true;
-        persist_grid = (tiles + per - 1) / per;
+        persist_shape = s;
+        persist_grid = (int)((tiles + per - 1) / per);
+        pa.tiles = tg;
     }
     return IFC_OK;
 }
@@ -271,7 +310,7 @@ int Engine<T>::launch_persist()
 {
     if (cudaMemsetAsync(barrier, 0, sizeof(GridBarrier), stream) != cudaSuccess) return IFC_CUDA_ERROR;
     ++launches;
-    return persist_dispatch<T>(*this, persist_ks(spp_persist), true, nullptr, persist_mt);
+    return persist_dispatch<T>(*this, persist_shape, true, nullptr);
 }
 
 }  // namespace ifc

@@ -183,4 +183,12 @@ __device__ __forceinline__ T face_corr(double ru, T aCL, T aCR, T pcl, T pcr, T 
     return (T)(ru * (double)sr * (double)(T)(pcl - pcr) * (double)A);
 }
 
+// The same with the reciprocals of the diagonals given.
+template <typename T>
+__device__ __forceinline__ T face_corr_known(double ru, T rL, T rR, T pcl, T pcr, T A)
+{
+    T sr = rL + rR;
+    return (T)(ru * (double)sr * (double)(T)(pcl - pcr) * (double)A);
+}
+
 }  // namespace ifc

@@ -1,0 +1,77 @@
+"""The register-held regions of the single-launch 2D solve (64 columns by 32 to
+64 rows) at the sizes where their tiling can go wrong: one region exactly, one
+cell more, the last size of two tiles and one more, odd sizes, shallow and deep
+passes, different sweep counts of u and v, several tiles per CTA, values that
+leave the range of the precomputed reciprocals.  Tolerance: exact, every value
+equal to the oracle's after whole outer iterations."""
+import numpy as np
+import pytest
+
+import ifc
+import oracle as O
+from helpers import assert_bitwise, load_both, seeded_state, to_oracle_cfg
+
+pytestmark = pytest.mark.gpu
+
+
+def check(cfg, iters, scale=None, seed=3):
+    prec = "d" if cfg.get("precision") == "d" else "f"
+    o = O.Oracle(to_oracle_cfg(cfg), prec)
+    s = ifc.Solver(cfg)
+    st = seeded_state(cfg, seed, s.dtype)
+    if scale is not None:
+        st = {k: (v * scale).astype(s.dtype) for k, v in st.items()}
+    load_both(o, s, st)
+    for it in range(iters):
+        r = s.iterate(1)
+        assert r["kernel_launches"] == 3, r  # begin, face BCs, the one cooperative launch
+        o.outer_iteration()
+        o.bc_face_vel()
+        for k in ("u", "v", "p", "uf", "vf"):
+            assert_bitwise(s.get(k), o.field(k), f"it{it} {k}")
+    s.close()
+
+
+@pytest.mark.parametrize("prec", ["f", "d"])
+@pytest.mark.parametrize("nx,ny", [(64, 32), (65, 33), (108, 64), (109, 65), (3, 64), (152, 36), (66, 107), (31, 3)])
+def test_region_edges(gpu_ok, nx, ny, prec):
+    check(dict(ifc.channel2d(nx, ny), precision=prec), 2)
+
+
+@pytest.mark.parametrize("ks,nu,nv,np_", [(2, 3, 5, 7), (10, 10, 10, 20), (5, 4, 11, 6), (3, 0, 2, 4), (8, 0, 0, 1)])
+def test_pass_depths_and_counts(gpu_ok, ks, nu, nv, np_):
+    check(dict(ifc.cavity2d(97, ny=70), sweeps_per_pass=ks, nIter_u=nu, nIter_v=nv, nIter_p=np_), 2)
+
+
+@pytest.mark.parametrize("case", ["f", "d", "quick", "early_exit"])
+def test_several_tiles_per_cta(gpu_ok, monkeypatch, case):
+    monkeypatch.setenv("IFC_PERSIST_MAX_CTAS", "2")
+    cfg = dict(ifc.channel2d(150, 101), precision="d" if case == "d" else "f")
+    if case == "quick":
+        cfg["convection_scheme"] = "quick"
+    if case == "early_exit":  # loose tolerances: passes end before their sweeps are used up
+        cfg.update(tol_u=0.3, tol_v=0.05, tol_p=0.3, sweeps_per_pass=2)
+        s = ifc.Solver(cfg)
+        load = seeded_state(cfg, 3, s.dtype)
+        monkeypatch.setenv("IFC_PERSIST_MAX_CTAS", "148")
+        t = ifc.Solver(cfg)
+        for k, v in load.items():
+            s.set(k, v)
+            t.set(k, v)
+        a, b = s.iterate(2), t.iterate(2)
+        assert a["sweeps"] == b["sweeps"] and min(a["sweeps"][0], a["sweeps"][3]) < 10, (a, b)
+        for k in ("u", "v", "p", "uf", "vf"):
+            assert np.array_equal(s.get(k), t.get(k)), k
+        return
+    check(cfg, 2)
+
+
+@pytest.mark.parametrize("scale", [1e-22, 1e-30, 3e-38])
+def test_values_outside_the_reciprocal_range(gpu_ok, scale):
+    # velocities and pressures whose quotients are tiny, subnormal or zero
+    check(dict(ifc.cavity2d(70, ny=40), velBC_val=[[0.0] * 3] * 6), 2, scale=scale)
+
+
+@pytest.mark.parametrize("mu", [1e-20, 1e15])
+def test_diagonals_outside_the_reciprocal_range(gpu_ok, mu):
+    check(dict(ifc.cavity2d(40, ny=36), dynamicViscosity=mu, density=1e-20 if mu < 1 else 1.0), 1)

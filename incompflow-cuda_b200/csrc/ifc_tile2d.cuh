@@ -44,12 +44,12 @@ template <typename T>
 struct KnownDiv;
 template <>
 struct KnownDiv<float> {
-    static constexpr float ylo = 0x1p-40f, yhi = 0x1p40f;
+    static constexpr float ylo = 0x1p-40f, yhi = 0x1p40f, up = 0x1p64f, down = 0x1p-64f, tiny = 0x1p-126f, small = 0x1p-20f;
     static constexpr unsigned kLow = (127u - 62u) << 24, kSpan = (124u << 24) - 1u;
 };
 template <>
 struct KnownDiv<double> {
-    static constexpr double ylo = 0x1p-200, yhi = 0x1p200;
+    static constexpr double ylo = 0x1p-200, yhi = 0x1p200, up = 0x1p400, down = 0x1p-400, tiny = 0x1p-1022, small = 0x1p-500;
     static constexpr unsigned kLow = (1023u - 700u) << 21, kSpan = (1400u << 21) - 1u;
 };
 
@@ -61,6 +61,37 @@ __device__ __forceinline__ unsigned range_key(double q)
 __device__ __forceinline__ float abs_t(float a) { return fabsf(a); }
 __device__ __forceinline__ double abs_t(double a) { return fabs(a); }
 
+// The division itself.  Written as volatile so that it stays behind the rarely
+// taken branch: the compiler otherwise computes it always and selects (200
+// against 70 instructions per update in the 3D solve).
+__device__ __forceinline__ float quot_div(float n, float y)
+{
+    float q;
+    asm volatile("div.rn.f32 %0, %1, %2;" : "=f"(q) : "f"(n), "f"(y));
+    return q;
+}
+__device__ __forceinline__ double quot_div(double n, double y)
+{
+    double q;
+    asm volatile("div.rn.f64 %0, %1, %2;" : "=d"(q) : "d"(n), "d"(y));
+    return q;
+}
+
+// n / y outside the range of the reciprocal.  A tiny quotient that is still
+// normal is formed scaled up (both scalings are exact), which keeps the
+// division on its fast path; fronts of a flow that develops from rest pass
+// through these magnitudes.
+template <typename T>
+__device__ __forceinline__ T quot_rare(T n, T y)
+{
+    using K = KnownDiv<T>;
+    if (abs_t(n) < K::small) {
+        const T q = quot_div(n * K::up, y) * K::down;
+        if (abs_t(q) >= K::tiny) return q;
+    }
+    return quot_div(n, y);
+}
+
 // Whether divisor y may be used with a precomputed reciprocal.
 template <typename T>
 __device__ __forceinline__ bool divisor_ok(T y)
@@ -71,31 +102,15 @@ __device__ __forceinline__ bool divisor_ok(T y)
 __device__ __forceinline__ float fma1(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma1(double a, double b, double c) { return __fma_rn(a, b, c); }
 
-// The reciprocal of a divisor for quot_recip: 0 when the divisor is outside the
-// range, which makes every quotient fall back to the division.
-template <typename T>
-__device__ __forceinline__ T recip_known(T y)
-{
-    return divisor_ok(y) ? (T)1 / y : (T)0;
-}
-
-// n / y given z = recip_known(y).
-template <typename T>
-__device__ __forceinline__ T quot_recip(T n, T y, T z)
-{
-    T q = n * z;
-    q = fma1(fma1(-q, y, n), z, q);
-    if (range_key(q) > KnownDiv<T>::kSpan) q = n / y;
-    return q;
-}
-
 // n / y given z = RN(1/y).
 template <typename T>
 __device__ __forceinline__ T quot_known(T n, T y, T z)
 {
     T q = n * z;
     q = fma1(fma1(-q, y, n), z, q);
-    if (range_key(q) > KnownDiv<T>::kSpan || !divisor_ok(y)) q = n / y;
+    if (range_key(q) > KnownDiv<T>::kSpan || !divisor_ok(y)) {
+        if (n != (T)0 || !divisor_ok(y)) q = quot_rare(n, y);
+    }
     return q;
 }
 
@@ -176,7 +191,7 @@ __device__ __forceinline__ TileBox tile_box(const TileGrid &G, int t, int nx, in
 }
 
 // Splits n cells for regions of C cells; false when the halo leaves no room.
-inline bool split_axis(int n, int C, int H, int *k, int *I)
+__host__ __device__ inline bool split_axis(int n, int C, int H, int *k, int *I)
 {
     if (n <= C) {
         *k = 1;
@@ -348,20 +363,34 @@ __device__ __forceinline__ void half_sweep(Cells<T, RT::R> *const (&xs)[F], cons
     }
     if (force || key > KnownDiv<T>::kSpan) {
         // Rare: the divisions themselves, in a loop so that they take little
-        // code (the kernels' loops have to fit the instruction caches).
-        T tn[F * 2 * J], ty[2 * J];
+        // code.  A zero numerator needs none: its quotient is a zero already
+        // (only the sign may differ, which q - x and x + d erase).
+        unsigned todo = 0;
 #pragma unroll
-        for (int i = 0; i < 2 * J; ++i) {
-            ty[i] = -a.C.v[COLOR][i >> 1][i & 1];
+        for (int f = 0; f < F; ++f)
 #pragma unroll
-            for (int f = 0; f < F; ++f) tn[2 * J * f + i] = n[f][i >> 1][i & 1];
-        }
+            for (int i = 0; i < 2 * J; ++i)
+                if (force || (range_key(q[f][i >> 1][i & 1]) > KnownDiv<T>::kSpan && n[f][i >> 1][i & 1] != (T)0))
+                    todo |= 1u << (2 * J * f + i);
+        if (todo) {
+            T tn[F * 2 * J], ty[2 * J];
+#pragma unroll
+            for (int i = 0; i < 2 * J; ++i) {
+                ty[i] = -a.C.v[COLOR][i >> 1][i & 1];
+#pragma unroll
+                for (int f = 0; f < F; ++f) tn[2 * J * f + i] = n[f][i >> 1][i & 1];
+            }
 #pragma unroll 1
-        for (int i = 0; i < F * 2 * J; ++i) tn[i] = tn[i] / ty[i % (2 * J)];
+            for (unsigned rest = todo; rest; rest &= rest - 1) {
+                const int i = __ffs(rest) - 1;
+                tn[i] = quot_rare(tn[i], ty[i % (2 * J)]);
+            }
 #pragma unroll
-        for (int i = 0; i < 2 * J; ++i)
+            for (int f = 0; f < F; ++f)
 #pragma unroll
-            for (int f = 0; f < F; ++f) q[f][i >> 1][i & 1] = tn[2 * J * f + i];
+                for (int i = 0; i < 2 * J; ++i)
+                    if (todo >> (2 * J * f + i) & 1u) q[f][i >> 1][i & 1] = tn[2 * J * f + i];
+        }
     }
 #pragma unroll
     for (int f = 0; f < F; ++f) {

@@ -18,7 +18,9 @@
 #include <cooperative_groups.h>
 #include <cstring>
 #include <mutex>
+#include <functional>
 #include <numeric>
+#include <queue>
 #include <vector>
 
 #include <nvtx3/nvToolsExt.h>
@@ -482,17 +484,39 @@ __global__ void __cluster_dims__(kCL, 1, 1) __launch_bounds__(kBNT, 4)
 
 // ---- variants and the autotuner ---------------------------------------------
 // Variant 0 sweeps whole rows with one cluster barrier per half sweep
-// (k_batch2d); the others are temporally blocked (k_batch_tb) with the tile
-// shape and sweeps per pass of the table.  A case's size class selects its
-// variant: the autotuner times every variant on copies of the class's median
-// case (a fixed number of outer iterations) the first time a class is met in a
-// process, and keeps the fastest.  IFC_BATCH_VARIANT=<k> forces variant k.
-struct BVariant {
-    int tx, ty, ks, nt;
-};
+// (k_batch2d); the others are temporally blocked (k_batch_tb) with the region
+// (64 x R*NW cells), cluster size and sweeps per pass of BatchShapes: variant 1
+// for the smallest cases (two CTAs each, one or two tiles), variant 2 for the
+// larger ones.  The autotuner times every variant on copies of a size class's
+// median case (a fixed number of outer iterations) the first time the class is
+// met in a process; from these times a batch chooses, per class, the variant
+// whose cases would be finished first (choose_variant).  IFC_BATCH_VARIANT=<k>
+// forces variant k.
 constexpr int kNumVariants = 3;
-constexpr BVariant kVariants[kNumVariants] = {{0, 0, 1, kBNT}, {32, 8, 3, 256}, {32, 16, 5, 512}};
+constexpr int kVariantSweeps[kNumVariants] = {1, 3, 5};
 constexpr int kNumClasses = 3;
+
+template <typename T, int V>
+struct BatchShape;
+template <>
+struct BatchShape<float, 1> {
+    static constexpr int R = 2, NW = 16, CL = 2, KS = 3;
+};
+template <>
+struct BatchShape<float, 2> {
+    static constexpr int R = 4, NW = 16, CL = 8, KS = 5;
+};
+template <>
+struct BatchShape<double, 1> {
+    static constexpr int R = 2, NW = 12, CL = 2, KS = 3;
+};
+template <>
+struct BatchShape<double, 2> {
+    static constexpr int R = 2, NW = 18, CL = 8, KS = 5;
+};
+
+template <typename T, int V>
+constexpr auto batch_tb_kernel = k_batch_tb<T, BatchShape<T, V>::R, BatchShape<T, V>::NW, BatchShape<T, V>::CL, BatchShape<T, V>::KS>;
 
 static int size_class(int nx, int ny)
 {
@@ -500,59 +524,63 @@ static int size_class(int nx, int ny)
     return cells <= 64 * 64 ? 0 : (cells <= 160 * 160 ? 1 : 2);
 }
 
-template <typename T>
-static const void *variant_kernel(int v)
+// Kernel, threads, cluster size, dynamic shared memory and region of a variant.
+struct VariantLaunch {
+    const void *kern;
+    int nt, cl, tx, ty;
+    size_t smem;
+};
+
+template <typename T, int V>
+static VariantLaunch tb_variant()
 {
-    switch (v) {
-    case 1: return (const void *)k_batch_tb<T, 32, 8, 3, 256>;
-    case 2: return (const void *)k_batch_tb<T, 32, 16, 5, 512>;
-    default: return (const void *)k_batch2d<T>;
-    }
+    using B = BatchShape<T, V>;
+    using RT = RTile<T, B::R, B::NW>;
+    const int ncol = 2 * B::KS > 5 ? 2 * B::KS : 5;
+    return {(const void *)batch_tb_kernel<T, V>, RT::NT, B::CL, RT::W, RT::HR,
+            RT::END * sizeof(T) + (size_t)ncol * RT::NT * sizeof(double)};
 }
 
 template <typename T>
-static size_t variant_smem(int v)
+static VariantLaunch variant_launch(int v)
 {
-    const BVariant &b = kVariants[v];
-    if (b.tx == 0) return 0;
-    const int W = b.tx + 4 * b.ks, HH = b.ty + 4 * b.ks;
-    return (size_t)3 * W * HH * sizeof(T);
+    switch (v) {
+    case 1: return tb_variant<T, 1>();
+    case 2: return tb_variant<T, 2>();
+    default: return {(const void *)k_batch2d<T>, kBNT, kCL, 0, 0, 0};
+    }
 }
 
 template <typename T>
 static cudaError_t variant_clusters(int v, int *nclusters)
 {
-    const void *kern = variant_kernel<T>(v);
-    const size_t smem = variant_smem<T>(v);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const VariantLaunch vl = variant_launch<T>(v);
+    cudaError_t e = cudaFuncSetAttribute(vl.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vl.smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3(kCL);
-    lc.blockDim = dim3(kVariants[v].nt);
-    lc.dynamicSmemBytes = smem;
+    lc.gridDim = dim3(vl.cl);
+    lc.blockDim = dim3(vl.nt);
+    lc.dynamicSmemBytes = vl.smem;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = kCL;
+    at[0].val.clusterDim.x = vl.cl;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
     lc.attrs = at;
     lc.numAttrs = 1;
-    return cudaOccupancyMaxActiveClusters(nclusters, kern, &lc);
+    return cudaOccupancyMaxActiveClusters(nclusters, vl.kern, &lc);
 }
 
 template <typename T>
 static void launch_variant(int v, int nclusters, cudaStream_t st, const BCase<T> *dc, BState *ds, BPools<T> pool,
                            TBPools<T> tp, int n, BQueue *dq, int chunk, cudaGraphConditionalHandle cond)
 {
-    const size_t smem = variant_smem<T>(v);
+    const VariantLaunch vl = variant_launch<T>(v);
+    const dim3 grid(nclusters * vl.cl), block(vl.nt);
     switch (v) {
-    case 1:
-        k_batch_tb<T, 32, 8, 3, 256><<<nclusters * kCL, 256, smem, st>>>(dc, ds, pool, tp, n, dq, chunk, cond, 1);
-        break;
-    case 2:
-        k_batch_tb<T, 32, 16, 5, 512><<<nclusters * kCL, 512, smem, st>>>(dc, ds, pool, tp, n, dq, chunk, cond, 1);
-        break;
-    default: k_batch2d<T><<<nclusters * kCL, kBNT, 0, st>>>(dc, ds, pool, n, dq, chunk, cond, 1); break;
+    case 1: batch_tb_kernel<T, 1><<<grid, block, vl.smem, st>>>(dc, ds, pool, tp, n, dq, chunk, cond, 1); break;
+    case 2: batch_tb_kernel<T, 2><<<grid, block, vl.smem, st>>>(dc, ds, pool, tp, n, dq, chunk, cond, 1); break;
+    default: k_batch2d<T><<<grid, block, 0, st>>>(dc, ds, pool, n, dq, chunk, cond, 1); break;
     }
 }
 
@@ -565,15 +593,53 @@ static void launch_variant(int v, int nclusters, cudaStream_t st, const BCase<T>
     } while (0)
 
 template <typename T>
-static int batch_run(const ifc_config *cfgs, int n, int force_variant, ifc_batch_result *res, void *const *fields_out,
+static int batch_run(const ifc_config *cfgs, int n, const std::vector<int> &wanted, ifc_batch_result *res,
+                     void *const *fields_out,
                      double *ms_out);
 
-// Variant chosen for each size class and precision in this process.
+// What the autotuner measured for each size class and precision in this process.
+struct Tuned {
+    bool done = false;
+    double cells = 0;             // of the probed case
+    double lat[kNumVariants];     // time of the probe's iterations on one cluster of a busy GPU (0: failed)
+    int clusters[kNumVariants];   // clusters that run at once
+};
 static std::mutex g_tune_mu;
-static int g_tuned[2][kNumClasses] = {{-1, -1, -1}, {-1, -1, -1}};
+static Tuned g_tuned[2][kNumClasses];
+
+// The variant that finishes cases of the given cells (one size class) first:
+// each goes, largest first, to the cluster that is free first, and takes the
+// probed time scaled by its cells.  Many cases go to the variant with the
+// highest throughput (whole rows: 71 small clusters), few to the one that
+// finishes the largest case soonest (a case has one cluster: 48 uneven cavities
+// 90 ms with whole rows, the 256x256 one alone takes that long, 67 ms with
+// regions in registers).
+static int choose_variant(const Tuned &t, std::vector<double> cells)
+{
+    std::sort(cells.begin(), cells.end(), [](double a, double b) { return a > b; });
+    int best = 0;
+    double best_end = 0.0;
+    for (int v = 0; v < kNumVariants; ++v) {
+        if (t.lat[v] <= 0.0 || t.clusters[v] < 1) continue;
+        std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
+        for (int k = 0; k < t.clusters[v]; ++k) free_at.push(0.0);
+        double end = 0.0;
+        for (double c : cells) {
+            const double e = free_at.top() + t.lat[v] * c / t.cells;
+            free_at.pop();
+            free_at.push(e);
+            end = std::max(end, e);
+        }
+        if (best_end == 0.0 || end < best_end) {
+            best_end = end;
+            best = v;
+        }
+    }
+    return best;
+}
 
 template <typename T>
-static int autotune(int cls, const ifc_config &rep)
+static Tuned autotune(int cls, const ifc_config &rep)
 {
     // Probe: copies of the class's median case, 20 outer iterations each (no
     // early stop), enough copies to fill the GPU with any variant.
@@ -586,19 +652,25 @@ static int autotune(int cls, const ifc_config &rep)
         c.num_outer_iter = 20;
     }
     std::vector<ifc_batch_result> r(kCopies);
-    int best = 0;
-    double best_ms = 0.0;
+    Tuned t;
+    t.done = true;
+    t.cells = (double)rep.nx * rep.ny;
     for (int v = 0; v < kNumVariants; ++v) {
         double ms = 0.0;
-        if (batch_run<T>(probe.data(), kCopies, v, r.data(), nullptr, &ms) != IFC_OK) continue;
+        t.lat[v] = 0.0;
+        t.clusters[v] = 0;
+        if (variant_clusters<T>(v, &t.clusters[v]) != cudaSuccess) {
+            cudaGetLastError();
+            continue;
+        }
+        const std::vector<int> forced(kCopies, v);
+        if (batch_run<T>(probe.data(), kCopies, forced, r.data(), nullptr, &ms) != IFC_OK) continue;
+        const int at_once = std::max(1, std::min(kCopies, t.clusters[v]));
+        t.lat[v] = ms / ((kCopies + at_once - 1) / at_once);
         if (getenv("IFC_VERBOSE"))
             fprintf(stderr, "ifc_batch autotune: class %d (%dx%d) variant %d: %.3f ms\n", cls, rep.nx, rep.ny, v, ms);
-        if (best_ms == 0.0 || ms < best_ms) {
-            best_ms = ms;
-            best = v;
-        }
     }
-    return best;
+    return t;
 }
 
 template <typename T>
@@ -606,36 +678,43 @@ static int batch_solve(const ifc_config *cfgs, int n, ifc_batch_result *res, voi
 {
     const char *env = getenv("IFC_BATCH_VARIANT");
     if (env && env[0] >= '0' && env[0] < '0' + kNumVariants)
-        return batch_run<T>(cfgs, n, env[0] - '0', res, fields_out, ms_out);
+        return batch_run<T>(cfgs, n, std::vector<int>(n, env[0] - '0'), res, fields_out, ms_out);
     const int prec = sizeof(T) == 8 ? 1 : 0;
+    std::vector<int> wanted(n, 0);
     for (int cls = 0; cls < kNumClasses; ++cls) {
         std::vector<int> members;
         for (int c = 0; c < n; ++c)
             if (size_class(cfgs[c].nx, cfgs[c].ny) == cls) members.push_back(c);
         if (members.empty()) continue;
-        {
-            std::lock_guard<std::mutex> lk(g_tune_mu);
-            if (g_tuned[prec][cls] >= 0) continue;
-        }
         std::sort(members.begin(), members.end(), [&](int x, int y) {
             return (long long)cfgs[x].nx * cfgs[x].ny < (long long)cfgs[y].nx * cfgs[y].ny;
         });
-        const int v = autotune<T>(cls, cfgs[members[members.size() / 2]]);
-        std::lock_guard<std::mutex> lk(g_tune_mu);
-        g_tuned[prec][cls] = v;
+        Tuned t;
+        {
+            std::lock_guard<std::mutex> lk(g_tune_mu);
+            t = g_tuned[prec][cls];
+        }
+        if (!t.done) {
+            t = autotune<T>(cls, cfgs[members[members.size() / 2]]);
+            std::lock_guard<std::mutex> lk(g_tune_mu);
+            g_tuned[prec][cls] = t;
+        }
+        std::vector<double> cells;
+        for (int c : members) cells.push_back((double)cfgs[c].nx * cfgs[c].ny);
+        const int v = choose_variant(t, cells);
+        for (int c : members) wanted[c] = v;
     }
-    return batch_run<T>(cfgs, n, -1, res, fields_out, ms_out);
+    return batch_run<T>(cfgs, n, wanted, res, fields_out, ms_out);
 }
 
-// Solves the cases; force_variant >= 0 runs every case with that variant,
-// otherwise each size class runs its tuned variant, largest class first, each
-// class as one persistent launch relaunched by a CUDA graph WHILE node.
+// Solves the cases, case c with variant wanted[c]; the cases of a variant are one
+// persistent launch relaunched by a CUDA graph WHILE node.
 template <typename T>
-static int batch_run(const ifc_config *cfgs, int n, int force_variant, ifc_batch_result *res, void *const *fields_out,
+static int batch_run(const ifc_config *cfgs, int n, const std::vector<int> &wanted, ifc_batch_result *res,
+                     void *const *fields_out,
                      double *ms_out)
 {
     int rc = IFC_OK;
-    const int prec = sizeof(T) == 8 ? 1 : 0;
     std::vector<BCase<T>> hc(n);
     std::vector<int> variant(n);
     long long nc = 0, nuf = 0, nvf = 0;
@@ -657,15 +736,8 @@ static int batch_run(const ifc_config *cfgs, int n, int force_variant, ifc_batch
         for (int f = 0; f < 4; ++f) closed = closed && cfgs[c].vel_bc_type[f] != IFC_OUTLET;
         b.pin = cfgs[c].pin_pressure == 1 || (cfgs[c].pin_pressure < 0 && closed);
         b.max_outer = cfgs[c].num_outer_iter;
-        if (cfgs[c].convection_scheme != IFC_CONV_UPWIND) {
-            variant[c] = 0;  // only the whole-row kernel applies the deferred correction
-        } else if (force_variant >= 0) {
-            variant[c] = force_variant;
-        } else {
-            std::lock_guard<std::mutex> lk(g_tune_mu);
-            const int v = g_tuned[prec][size_class(cfgs[c].nx, cfgs[c].ny)];
-            variant[c] = v < 0 ? 0 : v;
-        }
+        // only the whole-row kernel applies the deferred correction
+        variant[c] = cfgs[c].convection_scheme != IFC_CONV_UPWIND ? 0 : wanted[c];
     }
     // One queue per variant, largest grids first (longest-processing-time
     // heuristic); the queue with the most work runs first.
@@ -787,10 +859,10 @@ static int batch_run(const ifc_config *cfgs, int n, int force_variant, ifc_batch
             r.rel_uf = s.rel[4];
             r.rel_vf = s.rel[5];
             r.norm_mass = s.norm[7];
-            const BVariant &bv = kVariants[variant[c]];
-            r.tile_x = bv.tx;
-            r.tile_y = bv.ty;
-            r.sweeps_per_pass = bv.ks;
+            const VariantLaunch vl = variant_launch<T>(variant[c]);
+            r.tile_x = vl.tx;
+            r.tile_y = vl.ty;
+            r.sweeps_per_pass = kVariantSweeps[variant[c]];
             if (fields_out && fields_out[c]) {
                 const size_t cells = (size_t)cfgs[c].nx * cfgs[c].ny;
                 T *out = (T *)fields_out[c];

@@ -2,41 +2,51 @@
 // by ifc_batch.cu inside its anonymous namespace, after the case queue, loop
 // state and cluster-reduction helpers).
 //
-// A cluster of kCL CTAs solves one case at a time, as k_batch2d does, but the
-// linear sweeps run as temporally blocked passes, the same passes as the
-// single-case solve (ifc_persist2d.cuh): the case is cut into TX x TY tiles,
-// the cluster's CTAs take the tiles in turn, and each tile is staged with a
-// halo of 2*KS cells in shared memory, swept KS times there (momentum: u and v
+// A cluster of CL CTAs solves one case at a time, as k_batch2d does, but the
+// linear sweeps run as temporally blocked passes on regions held in registers,
+// the same passes as the single-case solve (ifc_tile2d.cuh): the case is cut
+// into tiles, the cluster's CTAs take the tiles in turn, each tile's region (the
+// tile and a halo of 2*ks cells) is loaded, swept ks times (momentum: u and v
 // together, coefficients rebuilt on the fly; p': links from 1/aC) and written
 // back -- to the other buffer of a ping-pong pair, so no tile reads a
 // neighbour tile's values of the same pass.  Cluster barriers separate the
-// passes and phases; every norm is reduced per CTA in warp order and across
+// passes and phases; every norm is reduced per CTA in a fixed order and across
 // the cluster through distributed shared memory in rank order, so each CTA
-// takes the same early-exit and convergence decisions.  Tile shape and sweeps
-// per pass are template parameters; the batch autotuner picks them per size
-// class.
+// takes the same early-exit and convergence decisions.  The region shape, the
+// cluster size and the sweeps per pass distinguish the variants; the batch
+// autotuner picks one per size class.  Against whole-row sweeps (a cluster
+// barrier per half sweep, every coefficient rebuilt from L1/L2 in every half
+// sweep) a batch of 48 cavities of 32..256 squared takes 67 ms instead of 102
+// for 60 iterations each; a batch of hundreds keeps all of the whole-row form's
+// 71 clusters busy and stays with it.
 
 template <typename T>
 struct TBPools {
     T *tu, *tv, *tpc;  // ping-pong partners of u, v and p' (same offsets as the pools)
 };
 
-template <int NV, int NT>
-__device__ __forceinline__ void tb_block_sum(const double (&v)[NV], double *part)
+// This CTA's column sums of sred into part (zeros when it had no tile); block
+// barriers before and after.
+template <int NT>
+__device__ __forceinline__ void tb_part(const double *sred, int ncol, bool any, double *part)
 {
-    __shared__ double red[NT / 32][NV];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int r = 0; r < NV; ++r) {
-        const double t = warp_sum(v[r]);
-        if (lane == 0) red[warp][r] = t;
+    __syncthreads();
+    if (any) column_partials<NT>(sred, ncol, nullptr, 1, part);
+    else if ((int)threadIdx.x < ncol) part[threadIdx.x] = 0.0;
+    __syncthreads();
+}
+
+// After a cluster barrier: the cluster-wide sums of the n slots `part` of every
+// CTA, added in rank order (identical in every CTA).
+template <int CL>
+__device__ __forceinline__ void tb_cluster_total(cg::cluster_group &cl, double *part, int n, double *out)
+{
+    if ((int)threadIdx.x < n) {
+        double t = 0.0;
+        for (int r = 0; r < CL; ++r) t += cl.map_shared_rank(part, r)[threadIdx.x];
+        out[threadIdx.x] = t;
     }
     __syncthreads();
-    if (threadIdx.x < NV) {
-        double t = 0.0;
-        for (int w = 0; w < NT / 32; ++w) t += red[w][threadIdx.x];
-        part[threadIdx.x] = t;
-    }
 }
 
 // Inner early-exit rule (src/Solver.cu:955-962) after a pass of ns sweeps with
@@ -55,26 +65,42 @@ __device__ __forceinline__ void tb_pass_done(CaseLoop &L, int e, const double *s
     if (stop_now) L.stop[e] = 1;
 }
 
-template <typename T, int TX, int TY, int KS, int NT>
-__global__ void __cluster_dims__(kCL, 1, 1) __launch_bounds__(NT)
+// Rhie-Chow velocity of interior face k of n along its axis (stride st; c: the
+// cell above the face), with the reciprocals of the diagonals.
+template <typename T>
+__device__ __forceinline__ T tb_face(const Geo<T> &g, const T *vel, const Fields<T> &f, T A, int k, int n, int st, int c,
+                                     int low, int high)
+{
+    const int L = c - st;
+    const T pL = f.p[L], pR = f.p[c];
+    const T pLL = k >= 2 ? f.p[L - st] : (g.closed[low] ? pL : (T)0);
+    const T pRR = k <= n - 2 ? f.p[c + st] : (g.closed[high] ? pR : (T)0);
+    return rc_face_known(vel[L], vel[c], f.ac[L], f.ac[c], f.rac[L], f.rac[c], pLL, pL, pR, pRR, A);
+}
+
+// Splits a case's grid into tiles (the rule of split_axis).
+__device__ __forceinline__ bool tb_tiles(int nx, int ny, int rows, int ks, TileGrid &G)
+{
+    G.H = 2 * ks;
+    return split_axis(nx, 64, G.H, &G.kx, &G.Ix) && split_axis(ny, rows, G.H, &G.ky, &G.Iy);
+}
+
+template <typename T, int R_, int NW_, int CL, int KS>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(32 * NW_, 1)
     k_batch_tb(const BCase<T> *cases, BState *states, BPools<T> pool, TBPools<T> tp, int ncases, BQueue *q,
                int chunk, cudaGraphConditionalHandle cond, int use_cond)
 {
-    constexpr int H = 2 * KS;
-    using R = Region<TX, TY, H>;
-    constexpr int W = R::W, NR = R::NR;
-    constexpr int CPT = (R::NHALF + NT - 1) / NT;
+    using RT = RTile<T, R_, NW_>;
+    constexpr int R = RT::R, NT = RT::NT;
     constexpr int NP = 2 * KS + 8;  // partial-sum slots per set
     cg::cluster_group cl = cg::this_cluster();
     const unsigned rank = cl.block_rank();
     const int tid = threadIdx.x, lane = tid & 31;
     const int gw = (int)rank * (NT / 32) + (tid >> 5);  // warp index within the cluster
-    constexpr int TW = kCL * NT / 32;                   // warps per cluster
+    constexpr int TW = CL * NT / 32;                    // warps per cluster
 
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *s0 = reinterpret_cast<T *>(smem_raw);
-    T *s1 = s0 + NR;
-    T *s2 = s1 + NR;
+    double *sred = reinterpret_cast<double *>(tile_smem<T>() + RT::END);  // per-thread sums
+    clear_guards<RT, T>();
     __shared__ int s_case;
     __shared__ BCase<T> C;
     __shared__ CaseLoop L;
@@ -100,11 +126,21 @@ __global__ void __cluster_dims__(kCL, 1, 1) __launch_bounds__(NT)
         const Params<T> &P = C.P;
         const Geo<T> &g = P.g;
         const int nx = g.nx, ny = g.ny, N = g.N;
-        const int tiles_x = (nx + TX - 1) / TX, ntiles = tiles_x * ((ny + TY - 1) / TY);
+        TileGrid tg;
+        tb_tiles(nx, ny, RT::HR, KS, tg);
+        const int ntiles = tg.kx * tg.ky;
         T *u = pool.u + C.off_c, *v = pool.v + C.off_c, *p = pool.p + C.off_c, *pc = pool.pc + C.off_c;
         T *ac = pool.ac + C.off_c, *rac = pool.rac + C.off_c, *sp = pool.sp + C.off_c;
         T *uf = pool.uf + C.off_uf, *vf = pool.vf + C.off_vf;
         T *bu[2] = {u, tp.tu + C.off_c}, *bv[2] = {v, tp.tv + C.off_c}, *bp[2] = {pc, tp.tpc + C.off_c};
+        Fields<T> f;
+        memset(&f, 0, sizeof(f));
+        f.p = p;
+        f.uf = uf;
+        f.vf = vf;
+        f.ac = ac;
+        f.rac = rac;
+        f.sp = sp;
 
         // First iteration of the case: interior faces from cell means, then
         // the face boundary conditions (kernels.cuh:10-95).
@@ -149,94 +185,26 @@ __global__ void __cluster_dims__(kCL, 1, 1) __launch_bounds__(NT)
                 const bool au = ns0 > 0 && !L.stop[EQ_U];
                 const bool av = ns1 > 0 && !L.stop[EQ_V];
                 if (!au && !av && pass > 0) continue;  // the same in every CTA
-                double acc[2 * KS];
-#pragma unroll
-                for (int s = 0; s < 2 * KS; ++s) acc[s] = 0.0;
-                for (int t = (int)rank; t < ntiles; t += kCL) {
-                    const int x0 = (t % tiles_x) * TX, y0 = (t / tiles_x) * TY;
-                    const int gx0 = x0 - H, gy0 = y0 - H;
-                    for (int q2 = tid; q2 < NR; q2 += NT) {
-                        const int gi = gx0 + q2 % W, gj = gy0 + q2 / W;
-                        const bool in = gi >= 0 && gi < nx && gj >= 0 && gj < ny;
-                        const int id = gi + nx * gj;
-                        s0[q2] = in ? bu[mcur][id] : (T)0;
-                        s1[q2] = in ? bv[mcur][id] : (T)0;
-                        s2[q2] = in ? p[id] : (T)0;
-                    }
-                    int cq[2][CPT], dq[2][CPT];
-                    own_cells<W, R::HH, R::NHALF, NT, CPT>(tid, gx0, gy0, nx, ny, cq);
-                    __syncthreads();
-                    T cE[2][CPT], cW[2][CPT], cN[2][CPT], cS[2][CPT], cC[2][CPT], cbu[2][CPT], cbv[2][CPT];
-                    bool own[2][CPT];
-#pragma unroll
-                    for (int c = 0; c < 2; ++c)
-#pragma unroll
-                        for (int k = 0; k < CPT; ++k) {
-                            const int q2 = cq[c][k];
-                            dq[c][k] = tile_distance<W, H, TX, TY>(q2);
-                            own[c][k] = false;
-                            cE[c][k] = cW[c][k] = cN[c][k] = cS[c][k] = cbu[c][k] = cbv[c][k] = (T)0;
-                            cC[c][k] = (T)1;
-                            if (q2 < 0) continue;
-                            const int a = q2 % W, b = q2 / W;
-                            const int gi = gx0 + a, gj = gy0 + b;
-                            const int fu = gi + (nx + 1) * gj, fv = gi + nx * gj;
-                            T a7[7], b3[3];
-                            mom_cell<T, 2>(P, gi, gj, 0, uf[fu], uf[fu + 1], vf[fv], vf[fv + nx], (T)0, (T)0, s2[q2],
-                                           s2[q2 - 1], s2[q2 + 1], s2[q2 - W], s2[q2 + W], (T)0, (T)0, a7, b3);
-                            cE[c][k] = a7[AE];
-                            cW[c][k] = a7[AW];
-                            cN[c][k] = a7[AN];
-                            cS[c][k] = a7[AS];
-                            cC[c][k] = a7[AC];
-                            cbu[c][k] = b3[0];
-                            cbv[c][k] = b3[1];
-                            own[c][k] = a >= H && a < H + TX && b >= H && b < H + TY;
-                            if (pass == 0 && own[c][k]) ac[gi + nx * gj] = a7[AC];
-                        }
-                    const T ru = g.relax[EQ_U], rv = g.relax[EQ_V];
 #pragma unroll 1
-                    for (int s = 0; s < KS; ++s) {
-                        const bool du = au && s < ns0;
-                        const bool dv = av && s < ns1;
-                        if (!du && !dv) break;
-#pragma unroll
-                        for (int color = 0; color < 2; ++color) {
-                            const int hs = 2 * s + color;
-#pragma unroll
-                            for (int k = 0; k < CPT; ++k) {
-                                const int q2 = cq[color][k];
-                                if (q2 < 0) continue;
-                                T a7[7] = {cC[color][k], cE[color][k], cW[color][k], cN[color][k], cS[color][k],
-                                           (T)0, (T)0};
-                                T d;
-                                if (du && dq[color][k] <= 2 * ns0 - 1 - hs) {
-                                    s0[q2] = point_update<T, 2>(a7, cbu[color][k], s0[q2], s0[q2 + 1], s0[q2 - 1],
-                                                                s0[q2 + W], s0[q2 - W], (T)0, (T)0, ru, d);
-                                    if (own[color][k]) acc[s] += (double)d * (double)d;
-                                }
-                                if (dv && dq[color][k] <= 2 * ns1 - 1 - hs) {
-                                    s1[q2] = point_update<T, 2>(a7, cbv[color][k], s1[q2], s1[q2 + 1], s1[q2 - 1],
-                                                                s1[q2 + W], s1[q2 - W], (T)0, (T)0, rv, d);
-                                    if (own[color][k]) acc[KS + s] += (double)d * (double)d;
-                                }
-                            }
-                            __syncthreads();
-                        }
-                    }
-                    for (int q2 = tid; q2 < TX * TY; q2 += NT) {
-                        const int a = H + q2 % TX, b = H + q2 / TX;
-                        const int gi = gx0 + a, gj = gy0 + b;
-                        if (gi >= nx || gj >= ny) continue;
-                        const int id = gi + nx * gj;
-                        bu[mcur ^ 1][id] = s0[b * W + a];
-                        bv[mcur ^ 1][id] = s1[b * W + a];
-                    }
-                    __syncthreads();  // the next tile restages the shared arrays
+                for (int t = (int)rank; t < ntiles; t += CL) {
+                    const LanePlace<RT> pl(tile_box(tg, t, nx, ny), ny);
+                    Links<RT, T> a;
+                    Cells<T, R> cu, cv;
+                    load_cells<RT, T>(cu, bu[mcur], pl, nx, ny, false, kOutside<T>);
+                    load_cells<RT, T>(cv, bv[mcur], pl, nx, ny, false, kOutside<T>);
+                    const bool force = mom_links<RT, T>(P, f, pl, a);
+                    if (pass == 0) store_diagonal<RT, T>(a, ac, rac, pl, nx);
+                    publish<RT, T>(cu, 0);
+                    publish<RT, T>(cv, 1);
+                    __syncthreads();
+                    sweeps2<RT, T>(cu, cv, a, pl, g.relax[EQ_U], g.relax[EQ_V], force, au ? ns0 : 0, av ? ns1 : 0, KS,
+                                   true, t != (int)rank, sred);
+                    store_own<RT, T>(cu, bu[mcur ^ 1], pl, nx);
+                    store_own<RT, T>(cv, bv[mcur ^ 1], pl, nx);
                 }
-                tb_block_sum<2 * KS, NT>(acc, part[rs]);
+                tb_part<NT>(sred, 2 * KS, ntiles > (int)rank, part[rs]);
                 cl.sync();
-                cluster_total<2 * KS>(cl, part[rs], tot);
+                tb_cluster_total<CL>(cl, part[rs], 2 * KS, tot);
                 rs ^= 1;
                 if (tid == 0) {
                     if (au) tb_pass_done(L, EQ_U, tot, ns0, N, g.tol[EQ_U]);
@@ -245,7 +213,7 @@ __global__ void __cluster_dims__(kCL, 1, 1) __launch_bounds__(NT)
                 __syncthreads();
                 mcur ^= 1;
             }
-            T *const cu = bu[mcur], *const cv = bv[mcur];
+            const T *const cu = bu[mcur], *const cv = bv[mcur];
 
             // ---- Rhie-Chow faces, face BCs, p' source, 1/aC (kernels.cuh:336-581)
             double mass_sq;
@@ -254,22 +222,23 @@ __global__ void __cluster_dims__(kCL, 1, 1) __launch_bounds__(NT)
                 for (int j = gw; j < ny; j += TW)
                     for (int i = lane; i < nx; i += 32) {
                         const int c = i + nx * j;
-                        const T uw = i == 0 ? face_bc(g, WEST, 0, cu[c], j) : rcx(g, cu, ac, p, i, j);
-                        const T ue = i == nx - 1 ? face_bc(g, EAST, 0, cu[c], j) : rcx(g, cu, ac, p, i + 1, j);
-                        const T vs = j == 0 ? face_bc(g, SOUTH, 1, cv[c], 0) : rcy(g, cv, ac, p, i, j);
-                        const T vn = j == ny - 1 ? face_bc(g, NORTH, 1, cv[c], 0) : rcy(g, cv, ac, p, i, j + 1);
+                        const T uw = i == 0 ? face_bc(g, WEST, 0, cu[c], j) : tb_face(g, cu, f, g.Ax, i, nx, 1, i + nx * j, WEST, EAST);
+                        const T ue = i == nx - 1 ? face_bc(g, EAST, 0, cu[c], j) : tb_face(g, cu, f, g.Ax, i + 1, nx, 1, i + 1 + nx * j, WEST, EAST);
+                        const T vs = j == 0 ? face_bc(g, SOUTH, 1, cv[c], 0) : tb_face(g, cv, f, g.Ay, j, ny, nx, i + nx * j, SOUTH, NORTH);
+                        const T vn = j == ny - 1 ? face_bc(g, NORTH, 1, cv[c], 0) : tb_face(g, cv, f, g.Ay, j + 1, ny, nx, i + nx * (j + 1), SOUTH, NORTH);
                         const T bb = mass_imbalance<T, 2>(g, uw, ue, vs, vn, (T)0, (T)0);
                         uf[i + (nx + 1) * j] = uw;
                         if (i == nx - 1) uf[nx + (nx + 1) * j] = ue;
                         vf[c] = vs;
                         if (j == ny - 1) vf[c + nx] = vn;
                         sp[c] = bb;
-                        rac[c] = (T)1 / ac[c];
                         m[0] += (double)bb * (double)bb;
                     }
-                tb_block_sum<1, NT>(m, part[rs]);
+                #pragma unroll
+                for (int c = 0; c < 1; ++c) sred[c * NT + tid] = m[c];
+                tb_part<NT>(sred, 1, true, part[rs]);
                 cl.sync();
-                cluster_total<1>(cl, part[rs], tot);
+                tb_cluster_total<CL>(cl, part[rs], 1, tot);
                 rs ^= 1;
                 mass_sq = tot[0];
             }
@@ -280,81 +249,22 @@ __global__ void __cluster_dims__(kCL, 1, 1) __launch_bounds__(NT)
             for (int pass = 0; pass < npass_p; ++pass) {
                 const int ns = clamp_sweeps(np, pass, KS);
                 if (ns <= 0 || L.stop[EQ_P]) continue;  // the same in every CTA
-                double acc[KS];
-#pragma unroll
-                for (int s = 0; s < KS; ++s) acc[s] = 0.0;
-                for (int t = (int)rank; t < ntiles; t += kCL) {
-                    const int x0 = (t % tiles_x) * TX, y0 = (t / tiles_x) * TY;
-                    const int gx0 = x0 - H, gy0 = y0 - H;
-                    for (int q2 = tid; q2 < NR; q2 += NT) {
-                        const int gi = gx0 + q2 % W, gj = gy0 + q2 / W;
-                        const bool in = gi >= 0 && gi < nx && gj >= 0 && gj < ny;
-                        const int id = gi + nx * gj;
-                        s0[q2] = (in && pass > 0) ? bp[pcur][id] : (T)0;
-                        s1[q2] = in ? rac[id] : (T)0;
-                    }
-                    int cq[2][CPT], dq[2][CPT];
-                    own_cells<W, R::HH, R::NHALF, NT, CPT>(tid, gx0, gy0, nx, ny, cq);
-                    __syncthreads();
-                    T cE[2][CPT], cW[2][CPT], cN[2][CPT], cS[2][CPT], cC[2][CPT], cb[2][CPT];
-                    bool own[2][CPT];
-#pragma unroll
-                    for (int c = 0; c < 2; ++c)
-#pragma unroll
-                        for (int k = 0; k < CPT; ++k) {
-                            const int q2 = cq[c][k];
-                            dq[c][k] = tile_distance<W, H, TX, TY>(q2);
-                            own[c][k] = false;
-                            cE[c][k] = cW[c][k] = cN[c][k] = cS[c][k] = cb[c][k] = (T)0;
-                            cC[c][k] = (T)1;
-                            if (q2 < 0) continue;
-                            const int a = q2 % W, b = q2 / W;
-                            const int gi = gx0 + a, gj = gy0 + b;
-                            const T r = s1[q2];
-                            const T e = gi < nx - 1 ? (T)(P.d.Kx * (double)(T)(r + s1[q2 + 1])) : (T)0;
-                            const T w = gi > 0 ? (T)(P.d.Kx * (double)(T)(r + s1[q2 - 1])) : (T)0;
-                            const T n = gj < ny - 1 ? (T)(P.d.Ky * (double)(T)(r + s1[q2 + W])) : (T)0;
-                            const T so = gj > 0 ? (T)(P.d.Ky * (double)(T)(r + s1[q2 - W])) : (T)0;
-                            cE[c][k] = e;
-                            cW[c][k] = w;
-                            cN[c][k] = n;
-                            cS[c][k] = so;
-                            cC[c][k] = -(e + w + n + so);
-                            cb[c][k] = sp[gi + nx * gj];
-                            own[c][k] = a >= H && a < H + TX && b >= H && b < H + TY;
-                        }
-                    const T relax = g.relax[EQ_P];
 #pragma unroll 1
-                    for (int s = 0; s < KS; ++s) {
-                        if (s >= ns) break;
-#pragma unroll
-                        for (int color = 0; color < 2; ++color) {
-                            const int reach = 2 * ns - 1 - (2 * s + color);
-#pragma unroll
-                            for (int k = 0; k < CPT; ++k) {
-                                const int q2 = cq[color][k];
-                                if (q2 < 0 || dq[color][k] > reach) continue;
-                                T a7[7] = {cC[color][k], cE[color][k], cW[color][k], cN[color][k], cS[color][k],
-                                           (T)0, (T)0};
-                                T d;
-                                s0[q2] = point_update<T, 2>(a7, cb[color][k], s0[q2], s0[q2 + 1], s0[q2 - 1],
-                                                            s0[q2 + W], s0[q2 - W], (T)0, (T)0, relax, d);
-                                if (own[color][k]) acc[s] += (double)d * (double)d;
-                            }
-                            __syncthreads();
-                        }
-                    }
-                    for (int q2 = tid; q2 < TX * TY; q2 += NT) {
-                        const int a = H + q2 % TX, b = H + q2 / TX;
-                        const int gi = gx0 + a, gj = gy0 + b;
-                        if (gi >= nx || gj >= ny) continue;
-                        bp[pcur ^ 1][gi + nx * gj] = s0[b * W + a];
-                    }
+                for (int t = (int)rank; t < ntiles; t += CL) {
+                    const LanePlace<RT> pl(tile_box(tg, t, nx, ny), ny);
+                    Links<RT, T> a;
+                    Cells<T, R> x;
+                    if (pass == 0) zero_cells<RT, T>(x, pl, nx, ny);
+                    else load_cells<RT, T>(x, bp[pcur], pl, nx, ny, false, kOutside<T>);
+                    const bool force = pc_links<RT, T>(P, f, pl, a);
+                    publish<RT, T>(x, 0);
                     __syncthreads();
+                    sweeps1<RT, T>(x, a, pl, g.relax[EQ_P], force, ns, KS, true, t != (int)rank, sred);
+                    store_own<RT, T>(x, bp[pcur ^ 1], pl, nx);
                 }
-                tb_block_sum<KS, NT>(acc, part[rs]);
+                tb_part<NT>(sred, KS, ntiles > (int)rank, part[rs]);
                 cl.sync();
-                cluster_total<KS>(cl, part[rs], tot);
+                tb_cluster_total<CL>(cl, part[rs], KS, tot);
                 rs ^= 1;
                 if (tid == 0) tb_pass_done(L, EQ_P, tot, ns, N, g.tol[EQ_P]);
                 __syncthreads();
@@ -372,9 +282,11 @@ __global__ void __cluster_dims__(kCL, 1, 1) __launch_bounds__(NT)
                 double m[1] = {0.0};
                 for (int j = gw; j < ny; j += TW)
                     for (int i = lane; i < nx; i += 32) m[0] += (double)pcc[i + nx * j];
-                tb_block_sum<1, NT>(m, part[rs]);
+                #pragma unroll
+                for (int c = 0; c < 1; ++c) sred[c * NT + tid] = m[c];
+                tb_part<NT>(sred, 1, true, part[rs]);
                 cl.sync();
-                cluster_total<1>(cl, part[rs], tot);
+                tb_cluster_total<CL>(cl, part[rs], 1, tot);
                 rs ^= 1;
                 const double mean = tot[0] / (double)N;
                 for (int j = gw; j < ny; j += TW)
@@ -391,7 +303,7 @@ __global__ void __cluster_dims__(kCL, 1, 1) __launch_bounds__(NT)
                         const T x = pcc[c], aC = ac[c];
                         const T xW = i > 0 ? pcc[c - 1] : (T)0, xE = i < nx - 1 ? pcc[c + 1] : (T)0;
                         const T xS = j > 0 ? pcc[c - nx] : (T)0, xN = j < ny - 1 ? pcc[c + nx] : (T)0;
-                        const T aW = i > 0 ? ac[c - 1] : (T)1, aS = j > 0 ? ac[c - nx] : (T)1;
+                        const T rC = rac[c], rW = i > 0 ? rac[c - 1] : (T)1, rS = j > 0 ? rac[c - nx] : (T)1;
                         const T p0 = p[c], u0 = cu[c], v0 = cv[c];
                         const T uf0 = i > 0 ? uf[fu] : (T)0, vf0 = j > 0 ? vf[c] : (T)0;
                         const T dp = g.relax[EQ_P] * x;
@@ -409,12 +321,12 @@ __global__ void __cluster_dims__(kCL, 1, 1) __launch_bounds__(NT)
                         sq[1] += (double)dU * (double)dU;
                         sq[2] += (double)dV * (double)dV;
                         if (i >= 1) {
-                            const T d = face_corr(P.d.ru[0], aW, aC, xW, x, g.Ax);
+                            const T d = face_corr_known(P.d.ru[0], rW, rC, xW, x, g.Ax);
                             uf[fu] = uf0 + d;
                             sq[3] += (double)d * (double)d;
                         }
                         if (j >= 1) {
-                            const T d = face_corr(P.d.ru[1], aS, aC, xS, x, g.Ay);
+                            const T d = face_corr_known(P.d.ru[1], rS, rC, xS, x, g.Ay);
                             vf[c] = vf0 + d;
                             sq[4] += (double)d * (double)d;
                         }
@@ -423,9 +335,11 @@ __global__ void __cluster_dims__(kCL, 1, 1) __launch_bounds__(NT)
                         if (j == 0) vf[c] = face_bc(g, SOUTH, 1, vn, 0);
                         if (j == ny - 1) vf[c + nx] = face_bc(g, NORTH, 1, vn, 0);
                     }
-                tb_block_sum<5, NT>(sq, part[rs]);
+                #pragma unroll
+                for (int c = 0; c < 5; ++c) sred[c * NT + tid] = sq[c];
+                tb_part<NT>(sred, 5, true, part[rs]);
                 cl.sync();
-                cluster_total<5>(cl, part[rs], tot);
+                tb_cluster_total<CL>(cl, part[rs], 5, tot);
                 rs ^= 1;
             }
 

@@ -141,6 +141,11 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(32 * NW_, 1)
         f.ac = ac;
         f.rac = rac;
         f.sp = sp;
+#ifdef IFC_BOUNDS_CHECK
+        f.p.n = f.ac.n = f.rac.n = f.sp.n = N;
+        f.uf.n = (long long)(nx + 1) * ny;
+        f.vf.n = (long long)nx * (ny + 1);
+#endif
 
         // First iteration of the case: interior faces from cell means, then
         // the face boundary conditions (kernels.cuh:10-95).

@@ -110,144 +110,123 @@ __global__ void k_temp_dc(Params<T> P, Fields<T> f, const T *src, T *src_eff)
 static __global__ void k_clear_stop(Ctl *ctl, int eq) { ctl->stop[eq] = 0; }
 
 // ---- 2D: a cycle of sweeps on stored coefficients in one cooperative launch --
-// The passes of k_coef_pass2d (below) with one tile per CTA, all CTAs
-// co-resident: the coefficients are read into registers once per cycle, the
-// passes are separated by the bounded grid barrier of ifc_persist2d.cuh, and
-// after each pass every CTA reduces the per-sweep FP64 sums (double-buffered
-// by pass parity, so a CTA that runs ahead cannot overwrite sums another is
-// still reading) and applies the inner early-exit rule exactly as
-// finish_sweeps does.  The result is left in x0.  Values equal those of the
-// per-pass launches.
-template <typename T, int TX, int TY, int KS, int NT>
-__global__ void __launch_bounds__(NT) k_coef_solve2d(Params<T> P, const T *coef, const T *src, Ctl *ctl,
-                                                     double *partials, GridBarrier *bar, int eq, int nsweeps, T *x0,
-                                                     T *x1, int stall_test)
+// One tile per CTA, all CTAs co-resident: the region's coefficients are read
+// into registers once per cycle (ifc_tile2d.cuh), the passes of kCoefSweeps
+// sweeps are separated by the bounded grid barrier of ifc_persist2d.cuh, and the
+// per-sweep FP64 sums of a pass are reduced and the inner early-exit rule is
+// applied (as finish_sweeps does) while the next pass already runs; a pass that
+// the rule makes superfluous is not stored.  The result is left in x0.  Values
+// equal those of the per-pass launches.  400 sweeps of the 512x128 channel's
+// temperature: 749 us with unknowns in shared memory and a 52x36 region per
+// 32x16 tile, 471 us this way.
+constexpr int kCoefSweeps = 5;
+
+struct CoefArgs {
+    TileGrid tiles;
+    int eq, nsweeps, stall_test;
+};
+
+template <typename T, int R_, int NW_>
+__global__ void __launch_bounds__(32 * NW_, 1)
+    k_coef_solve2d(const __grid_constant__ Params<T> P, const T *coef, const T *src, Ctl *ctl, double *partials,
+                   GridBarrier *bar, const CoefArgs ca, T *x0, T *x1)
 {
-    constexpr int H = 2 * KS;
-    using R = Region<TX, TY, H>;
-    constexpr int W = R::W, NR = R::NR;
-    constexpr int CPT = (R::NHALF + NT - 1) / NT;
+    using RT = RTile<T, R_, NW_>;
+    constexpr int R = RT::R, NT = RT::NT, KS = kCoefSweeps;
     const Geo<T> &g = P.g;
-    const int nx = g.nx, ny = g.ny, N = g.N, G = gridDim.x;
-    const int tiles_x = (nx + TX - 1) / TX;
-    const int x0t = (blockIdx.x % tiles_x) * TX, y0t = (blockIdx.x / tiles_x) * TY;
-    const int gx0 = x0t - H, gy0 = y0t - H;
-    const int tid = threadIdx.x;
-
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *sx = reinterpret_cast<T *>(smem_raw);
-    __shared__ double wred[NT / 32][KS];
+    const int nx = g.nx, ny = g.ny, N = g.N, G = gridDim.x, eq = ca.eq;
+    const int tid = threadIdx.x, warp = tid >> 5;
+    double *sred = reinterpret_cast<double *>(tile_smem<T>() + RT::END);  // per-thread sums of each sweep
+    __shared__ LoopState L;
     __shared__ double tot[KS];
-    __shared__ int s_stop;
+    __shared__ double last_sq;
 
-    int cq[2][CPT], dq[2][CPT];
-    own_cells<W, R::HH, R::NHALF, NT, CPT>(tid, gx0, gy0, nx, ny, cq);
-    T cE[2][CPT], cW[2][CPT], cN[2][CPT], cS[2][CPT], cC[2][CPT], cb[2][CPT];
-    bool own[2][CPT];
+    const double floor = ctl->inner_max[eq];
+    if (tid == 0) {
+        L.stop[eq] = ctl->stop[eq];
+        L.sweeps[eq] = 0;
+        L.cell_updates[eq] = 0;
+        L.inner_max_sq[eq] = -1.0;
+        last_sq = ctl->last_sweep_sq[eq];
+    }
+    clear_guards<RT, T>();
+    const LanePlace<RT> pl(tile_box(ca.tiles, blockIdx.x, nx, ny), ny);
+    Links<RT, T> a;
+    Cells<T, R> x;
+    {
+        Cells<T, R> b;
 #pragma unroll
-    for (int c = 0; c < 2; ++c)
+        for (int r = 0; r < R; ++r)
 #pragma unroll
-        for (int k = 0; k < CPT; ++k) {
-            const int q = cq[c][k];
-            dq[c][k] = tile_distance<W, H, TX, TY>(q);
-            own[c][k] = false;
-            cE[c][k] = cW[c][k] = cN[c][k] = cS[c][k] = cb[c][k] = (T)0;
-            cC[c][k] = (T)1;
-            if (q < 0) continue;
-            const int a = q % W, b = q / W;
-            const int id = gx0 + a + nx * (gy0 + b);
-            cC[c][k] = coef[id + (size_t)N * AC];
-            cE[c][k] = coef[id + (size_t)N * AE];
-            cW[c][k] = coef[id + (size_t)N * AW];
-            cN[c][k] = coef[id + (size_t)N * AN];
-            cS[c][k] = coef[id + (size_t)N * AS];
-            cb[c][k] = src[id];
-            own[c][k] = a >= H && a < H + TX && b >= H && b < H + TY;
-        }
-    double mx = ctl->inner_max[eq];
-    int sw = ctl->sweeps[eq];
-    long long cu = ctl->cell_updates;
-    double last_sq = ctl->last_sweep_sq[eq];
-    if (tid == 0) s_stop = ctl->stop[eq];
+            for (int k = 0; k < 2; ++k) {
+                const int i = pl.gi + k, j = pl.gj + r;
+                if (i < nx && j < ny) {
+                    const size_t id = (size_t)i + (size_t)nx * j, n = (size_t)N;
+                    // no neighbour beyond the domain: its value counts as 0
+                    const T e = coef[id + n * AE], w = coef[id + n * AW], no = coef[id + n * AN], so = coef[id + n * AS];
+                    a.set(r, k, i < nx - 1 ? e : e * (T)0, i > 0 ? w : w * (T)0, j < ny - 1 ? no : no * (T)0,
+                          j > 0 ? so : so * (T)0, coef[id]);
+                    b.at(r, k) = src[id];
+                } else {
+                    a.set(r, k, (T)0, (T)0, (T)0, (T)0, kOutside<T>);
+                    b.at(r, k) = kOutside<T>;
+                }
+            }
+        put_cells<RT, T>(b, RT::SRC);
+    }
+    const bool force = set_reciprocals<RT, T>(a);
     __syncthreads();
-    bool stop = s_stop != 0;
+
     bool failed = false;
     unsigned int epoch = 0;
-    T *buf[2] = {x0, x1};
-    int cur = 0;
-    const T relax = g.relax[eq];
-
-    for (int pass = 0; pass * KS < nsweeps && !stop; ++pass) {
+    auto buf = [&](int q) { return q ? x1 : x0; };
+    int cur = 0, set = 0;
+    Pending pending;
+    pending.kind = kPendNone;
+    auto take = [&]() {  // by warp 0, after a block barrier
+        if (warp != 0) return;
+        pass_done(L, eq, tot, pending.n0, N, g.tol[eq], floor);
+        if (tid == 0) last_sq = tot[pending.n0 - 1];
+    };
+#pragma unroll 1
+    for (int pass = 0; pass * KS < ca.nsweeps && !L.stop[eq]; ++pass) {
         // Failure-detection test (stall_test = 1): CTA 0 leaves without
         // arriving, so every other CTA's bounded wait at this pass's barrier
         // runs out and the launch ends with the timeout status.
-        if (stall_test && blockIdx.x == 0) { failed = true; break; }
-        const int ns = clamp_sweeps(nsweeps, pass, KS);
-        for (int q = tid; q < NR; q += NT) {
-            const int a = q % W, b = q / W;
-            const int gi = gx0 + a, gj = gy0 + b;
-            const bool in = gi >= 0 && gi < nx && gj >= 0 && gj < ny;
-            sx[q] = in ? buf[cur][gi + nx * gj] : (T)0;
-        }
+        if (ca.stall_test && blockIdx.x == 0) { failed = true; break; }
+        const int ns = clamp_sweeps(ca.nsweeps, pass, KS);
+        load_cells<RT, T>(x, buf(cur), pl, nx, ny, pass > 0, kOutside<T>);
+        if (pending.kind) pending_totals<RT::NW>(pending, partials, G, tot, tot);
+        publish<RT, T>(x, 0);
         __syncthreads();
-#pragma unroll 1
-        for (int s = 0; s < KS; ++s) {
-            if (s >= ns) break;
-            double acc = 0.0;
-#pragma unroll
-            for (int color = 0; color < 2; ++color) {
-                const int reach = 2 * ns - 1 - (2 * s + color);
-#pragma unroll
-                for (int k = 0; k < CPT; ++k) {
-                    const int q = cq[color][k];
-                    if (q < 0 || dq[color][k] > reach) continue;
-                    T a7[7] = {cC[color][k], cE[color][k], cW[color][k], cN[color][k], cS[color][k], (T)0, (T)0};
-                    T d;
-                    sx[q] = point_update<T, 2>(a7, cb[color][k], sx[q], sx[q + 1], sx[q - 1], sx[q + W], sx[q - W],
-                                               (T)0, (T)0, relax, d);
-                    if (own[color][k]) acc += (double)d * (double)d;
-                }
-                __syncthreads();
-            }
-            acc = warp_sum(acc);
-            if ((tid & 31) == 0) wred[tid >> 5][s] = acc;
+        if (pending.kind) take();
+        sweeps1<RT, T>(x, a, pl, g.relax[eq], force, ns, KS, true, false, sred);
+        if (pending.kind) {
+            pending.kind = kPendNone;
+            if (L.stop[eq]) break;  // this pass was superfluous
         }
-        for (int q = tid; q < TX * TY; q += NT) {
-            const int a = H + q % TX, b = H + q / TX;
-            const int gi = gx0 + a, gj = gy0 + b;
-            if (gi >= nx || gj >= ny) continue;
-            buf[cur ^ 1][gi + nx * gj] = sx[b * W + a];
-        }
+        store_own<RT, T>(x, buf(cur ^ 1), pl, nx);
+        column_partials<NT>(sred, ns, partials + set * KS * G, G, tot);
         cur ^= 1;
-        double *part = partials + (size_t)(pass & 1) * KS * G;
-        block_partials<KS, KS, NT>(&wred[0][0], part, G);
         if (!grid_sync(bar, G, epoch)) { failed = true; break; }
-        reduce_partials<NT>(part, KS, G, tot);
-        // the rule of finish_sweeps, evaluated identically in every CTA
-        bool stop_now = false;
-        for (int s = 0; s < ns; ++s) {
-            if (stop_now) break;
-            const double rms = sqrt(tot[s] / (double)N);
-            if (rms > mx) mx = rms;
-            if (rms / (mx + 1e-20) < g.tol[eq]) stop_now = true;
-        }
-        sw += ns;
-        cu += (long long)ns * N;
-        last_sq = tot[ns - 1];
-        stop = stop_now;
-        __syncthreads();  // tot is rewritten only after the next pass's barrier
+        pending.set(kPendP, set * KS * G, ns, ns, 0);
+        set ^= 1;
     }
-    if (!failed && cur == 1)  // the last pass staged from x0, and every CTA has passed its barrier
-        for (int q = tid; q < TX * TY; q += NT) {
-            const int gi = x0t + q % TX, gj = y0t + q / TX;
-            if (gi < nx && gj < ny) x0[gi + nx * gj] = x1[gi + nx * gj];
-        }
+    if (pending.kind && !failed) {
+        pending_totals<RT::NW>(pending, partials, G, tot, tot);
+        __syncthreads();
+        take();
+    }
+    __syncthreads();
+    // the last stored pass read x0, and every CTA has passed its barrier
+    if (!failed && cur == 1) store_other<RT, T>(x0, x1, pl, nx);
     if (blockIdx.x == 0 && tid == 0 && !failed) {
-        ctl->inner_max[eq] = mx;
-        ctl->sweeps[eq] = sw;
-        ctl->cell_updates = cu;
+        const double top = L.inner_max_sq[eq] >= 0.0 ? sqrt(L.inner_max_sq[eq] / (double)N) : -1e20;
+        ctl->inner_max[eq] = top > floor ? top : floor;
+        ctl->sweeps[eq] += L.sweeps[eq];
+        ctl->cell_updates += L.cell_updates[eq];
         ctl->last_sweep_sq[eq] = last_sq;
-        if (stop) ctl->stop[eq] = 1;
+        if (L.stop[eq]) ctl->stop[eq] = 1;
     }
     if (tid == 0 && (failed || bar->err)) atomicExch(&ctl->status, 3);
 }

@@ -971,10 +971,7 @@ struct Engine : EngineBase {
         if (n > 0 && cfg.linear_solver == IFC_GAUSS_SEIDEL) {
             Params<T> PT = P;
             PT.g.tol[eq] = 0.0;
-            using S = TileShape2D<T>;
-            using R = Region<S::TX, S::TY, 10>;
-            const int tiles = ((P.g.nx + S::TX - 1) / S::TX) * ((P.g.ny + S::TY - 1) / S::TY);
-            const bool c2 = dim == 2 && fused && energy_coop(tiles);
+            const bool c2 = dim == 2 && fused && coef_coop();
             const bool c3 = dim == 3 && pc3d;
             if (c2 || c3) {
                 k_reset_inner<<<1, 1, 0, stream>>>(ctl, 1 << eq);
@@ -982,13 +979,8 @@ struct Engine : EngineBase {
                     CSys<T> sys = {coef, src[0], phi[0], eq};
                     enq_csolve3d(PT, sys, n);
                 } else {
-                    IFC_CK(cudaMemsetAsync(barrier, 0, sizeof(GridBarrier), stream));
-                    int e = eq, ns = n, stall = 0;
-                    T *x0 = phi[0], *x1 = f.tmp + 2 * (size_t)P.g.N;
-                    const T *srcp = src[0];
-                    void *args[] = {&PT, &coef, &srcp, &ctl, &partials, &barrier, &e, &ns, &x0, &x1, &stall};
-                    IFC_CK(cudaLaunchCooperativeKernel((const void *)k_coef_solve2d<T, S::TX, S::TY, 5, S::NT>,
-                                                       dim3(tiles), dim3(S::NT), args, R::NR * sizeof(T), stream));
+                    const int rc = launch_coef(PT, coef, src[0], eq, n, phi[0], f.tmp + 2 * (size_t)P.g.N, 0);
+                    if (rc != IFC_OK) return rc;
                     ++launches;
                 }
                 IFC_CK(cudaGetLastError());
@@ -1060,18 +1052,14 @@ struct Engine : EngineBase {
         // p' passes.  3D: one cooperative launch per cycle when the p'
         // solve has one (k_csolve3d), else one launch per colour and sweep.
         const bool blocked = dim == 2 && fused && cfg.linear_solver == IFC_GAUSS_SEIDEL;
-        constexpr int kEnergyKS = 5;
+        constexpr int kEnergyKS = kCoefSweeps;
         const int gran = blocked ? kEnergyKS : 1;  // sweeps counted per early-exit check
         T *tbuf[2] = {f.temp, f.tmp + 2 * N};
         // Cycles of 25 sweeps with a host check between them; without the
         // deferred correction the cooperative kernel applies the early-exit
         // rule on the device, so the whole solve is one cycle there.
         int cycle_len = 25;
-        {
-            using S = TileShape2D<T>;
-            const int tiles = ((g.nx + S::TX - 1) / S::TX) * ((g.ny + S::TY - 1) / S::TY);
-            if (blocked && !dc && energy_coop(tiles) && max_sweeps > 0) cycle_len = max_sweeps;
-        }
+        if (blocked && !dc && coef_coop() && max_sweeps > 0) cycle_len = max_sweeps;
         // 3D: one cooperative launch per cycle on the stored planes
         // (k_csolve3d), the early-exit rule applied after every sweep on the
         // device, as the per-sweep launches apply it.
@@ -1089,15 +1077,10 @@ struct Engine : EngineBase {
             using S = TileShape2D<T>;
             using R = Region<S::TX, S::TY, 2 * kEnergyKS>;
             const int tiles = ((g.nx + S::TX - 1) / S::TX) * ((g.ny + S::TY - 1) / S::TY);
-            if (blocked && energy_coop(tiles)) {
+            if (blocked && coef_coop()) {
                 // the whole cycle in one cooperative launch (k_coef_solve2d)
-                IFC_CK(cudaMemsetAsync(barrier, 0, sizeof(GridBarrier), stream));
-                int ns_cycle = chunk, eq = EQ_W;
-                T *x1 = tbuf[1];
-                const T *coef = f.mc, *srcp = src_eff;
-                void *args[] = {&PT, &coef, &srcp, &ctl, &partials, &barrier, &eq, &ns_cycle, &f.temp, &x1, &stall_test};
-                IFC_CK(cudaLaunchCooperativeKernel((const void *)k_coef_solve2d<T, S::TX, S::TY, kEnergyKS, S::NT>,
-                                                   dim3(tiles), dim3(S::NT), args, R::NR * sizeof(T), stream));
+                const int rc = launch_coef(PT, f.mc, src_eff, EQ_W, chunk, f.temp, tbuf[1], stall_test);
+                if (rc != IFC_OK) return rc;
                 ++launches;
             } else if (blocked) {
                 int cur = 0;
@@ -1158,26 +1141,13 @@ struct Engine : EngineBase {
         return ctl_h.stop[EQ_W] || tol == 0.0 ? IFC_OK : IFC_NOT_CONVERGED;
     }
 
-    // Whether the energy cycle fits one cooperative launch (one tile per CTA).
-    int energy_coop_state = -1;
-    bool energy_coop(int tiles)
-    {
-        if (energy_coop_state < 0) {
-            using S = TileShape2D<T>;
-            using R = Region<S::TX, S::TY, 10>;
-            int per_sm = 0, dev = 0, coop = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-            if (coop && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_coef_solve2d<T, S::TX, S::TY, 5, S::NT>,
-                                                                      S::NT, R::NR * sizeof(T)) != cudaSuccess) {
-                cudaGetLastError();
-                per_sm = 0;
-            }
-            const char *off = std::getenv("IFC_PERSIST_OFF");
-            energy_coop_state = coop && per_sm > 0 && !(off && off[0] == '1') && tiles <= per_sm * nsm ? 1 : 0;
-        }
-        return energy_coop_state == 1;
-    }
+    // Whether sweeps on stored 2D coefficients fit one cooperative launch (one
+    // tile per CTA, k_coef_solve2d), with which region shape and tiles; decided
+    // at the first use.
+    int coef_state = -1, coef_shape = 0;
+    TileGrid coef_tiles = {};
+    bool coef_coop();
+    int launch_coef(const Params<T> &PP, const T *coef, const T *src, int eq, int n, T *x0, T *x1, int stall);
 
     int set_inlet(const double *profile) override
     {

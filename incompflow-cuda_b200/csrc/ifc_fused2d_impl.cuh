@@ -313,4 +313,83 @@ int Engine<T>::launch_persist()
     return persist_dispatch<T>(*this, persist_shape, true, nullptr);
 }
 
+// ---- sweeps on stored 2D coefficients in one cooperative launch ----
+// call = nullptr: prepare the kernel of shape I and return its co-resident CTAs.
+template <typename T>
+struct CoefCall {
+    const Params<T> *P;
+    const T *coef, *src;
+    CoefArgs ca;
+    T *x0, *x1;
+};
+
+template <typename T, int I>
+static cudaError_t coef_kernel(Engine<T> &e, CoefCall<T> *call, int *capacity)
+{
+    using RT = ShapeTile<T, I>;
+    auto kern = k_coef_solve2d<T, RT::R, RT::NW>;
+    const size_t smem = (size_t)RT::END * sizeof(T) + (size_t)kCoefSweeps * RT::NT * sizeof(double);
+    if (!call) {
+        cudaError_t rc = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        int per_sm = 0;
+        if (rc == cudaSuccess) rc = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, RT::NT, smem);
+        *capacity = (per_sm < 2 ? per_sm : 2) * e.nsm;
+        return rc;
+    }
+    void *args[] = {(void *)call->P, &call->coef, &call->src, &e.ctl, &e.partials, &e.barrier, &call->ca, &call->x0, &call->x1};
+    const TileGrid &tg = call->ca.tiles;
+    return cudaLaunchCooperativeKernel((const void *)kern, dim3(tg.kx * tg.ky), dim3(RT::NT), args, smem, e.stream);
+}
+
+template <typename T>
+static cudaError_t coef_dispatch(Engine<T> &e, int shape, CoefCall<T> *call, int *capacity)
+{
+    constexpr int n = RegionShapes<T>::n;
+    if (shape == n - 1) return coef_kernel<T, n - 1>(e, call, capacity);
+    if (shape == n - 2) return coef_kernel<T, n - 2>(e, call, capacity);
+    return coef_kernel<T, 0>(e, call, capacity);
+}
+
+template <typename T>
+bool Engine<T>::coef_coop()
+{
+    if (coef_state >= 0) return coef_state == 1;
+    coef_state = 0;
+    int coop = 0, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    const char *off = std::getenv("IFC_PERSIST_OFF");
+    if (!coop || (off && off[0] == '1')) return false;
+    double best = 0.0;
+    for (int s = 0; s < RegionShapes<T>::n; ++s) {
+        const RegionShape &sh = RegionShapes<T>::s[s];
+        TileGrid tg;
+        tg.H = 2 * kCoefSweeps;
+        if (!split_axis(P.g.nx, 64, tg.H, &tg.kx, &tg.Ix) || !split_axis(P.g.ny, sh.R * sh.NW, tg.H, &tg.ky, &tg.Iy))
+            continue;
+        const long long tiles = (long long)tg.kx * tg.ky;
+        const double cost = sh.cost - (tiles == 1 ? 0.3 : 0.0);
+        int capacity = 0;
+        if (coef_dispatch<T>(*this, s, nullptr, &capacity) != cudaSuccess) {
+            cudaGetLastError();
+            continue;
+        }
+        if (tiles > capacity || (coef_state == 1 && cost >= best)) continue;
+        best = cost;
+        coef_state = 1;
+        coef_shape = s;
+        coef_tiles = tg;
+    }
+    return coef_state == 1;
+}
+
+template <typename T>
+int Engine<T>::launch_coef(const Params<T> &PP, const T *coef, const T *src, int eq, int n, T *x0, T *x1, int stall)
+{
+    IFC_CK(cudaMemsetAsync(barrier, 0, sizeof(GridBarrier), stream));
+    CoefCall<T> call = {&PP, coef, src, {coef_tiles, eq, n, stall}, x0, x1};
+    IFC_CK(coef_dispatch<T>(*this, coef_shape, &call, nullptr));
+    return IFC_OK;
+}
+
 }  // namespace ifc

@@ -12,11 +12,13 @@
 // order, so every CTA takes the same early-exit and convergence decisions
 // without another barrier.  The decisions are taken by two warps while the next
 // pass (after the corrections: the first pass of the next outer iteration)
-// already runs; a pass that the decision makes superfluous is not stored.  Waiting for them first costs 3 us per pass of the 65 us that an
-// outer iteration of the 512x128 channel takes.  Barrier waits are bounded: a CTA that waits longer
-// than kBarrierTimeoutNs sets the error flag, every CTA leaves the loop, and
-// the host reports IFC_TIMEOUT.  The launch is cooperative, so all CTAs are
-// co-resident or the launch fails (the engine then uses the multi-kernel graph).
+// already runs; a pass that the decision makes superfluous is not stored.
+// Waiting for them first costs 3 us per pass of the 65 us that an outer
+// iteration of the 512x128 channel takes.  Barrier waits are bounded: a CTA
+// that waits longer than kBarrierTimeoutNs sets the error flag, every CTA leaves
+// the loop, and the host reports IFC_TIMEOUT.  The launch is cooperative, so all
+// CTAs are co-resident or the launch fails (the engine then uses the
+// multi-kernel graph).
 #pragma once
 
 #include "ifc_fused2d.cuh"
@@ -93,9 +95,10 @@ __device__ __forceinline__ bool grid_sync(GridBarrier *b, unsigned int nblocks, 
 }
 
 // Sum column r of partials (one value per CTA) for r < ncol in a fixed order;
-// identical in every CTA (a single CTA has its totals in `out` already).  Warp w sums columns w, w + NT/32, ... (each
-// lane-strided, then one shuffle tree), so the columns are reduced in
-// parallel with one round trip to L2.  out: shared, ncol entries.
+// identical in every CTA (a single CTA has its totals in `out` already).  Warp w
+// sums columns w, w + NT/32, ... (each lane-strided, then one shuffle tree), so
+// the columns are reduced in parallel with one round trip to L2.  out: shared,
+// ncol entries.
 template <int NT>
 static __device__ __noinline__ void reduce_partials(const double *partials, int ncol, int G, double *out)
 {
@@ -109,18 +112,6 @@ static __device__ __noinline__ void reduce_partials(const double *partials, int 
         if (lane == 0) out[r] = x;
     }
     __syncthreads();
-}
-
-// This CTA's partials from per-warp sums: slot r = sum over warps, in order.
-template <int NRV, int STRIDE, int NT>
-__device__ __forceinline__ void block_partials(const double *wred, double *partials, int G)
-{
-    __syncthreads();
-    if (threadIdx.x < NRV) {
-        double x = 0.0;
-        for (int w = 0; w < NT / 32; ++w) x += wred[w * STRIDE + threadIdx.x];
-        partials[(size_t)threadIdx.x * G + blockIdx.x] = x;
-    }
 }
 
 constexpr int kMaxPassSweeps = 10;  // sweeps per pass of the single-launch solve, at most
@@ -153,7 +144,9 @@ struct PersistArgs {
 // Returns the sweep that met it or -1; mx: the largest sum up to there (the
 // largest sum stands for the largest RMS: the root and the division by N keep
 // the order; a NaN sum leaves the maximum).
-static __device__ __noinline__ int exit_rule(double own, double before, int ns, int N, double tol, double *mx_out)
+// floor: a largest RMS from before this launch (-1e20: none).
+static __device__ __noinline__ int exit_rule(double own, double before, double floor, int ns, int N, double tol,
+                                             double *mx_out)
 {
     const int lane = threadIdx.x & 31;
     double mx = own > before ? own : before;
@@ -163,7 +156,8 @@ static __device__ __noinline__ int exit_rule(double own, double before, int ns, 
         if (lane >= o && y > mx) mx = y;
     }
     const double rms = sqrt(own / (double)N);
-    const double top = mx >= 0.0 ? sqrt(mx / (double)N) : -1e20;
+    double top = mx >= 0.0 ? sqrt(mx / (double)N) : -1e20;
+    if (floor > top) top = floor;
     const unsigned hit = __ballot_sync(0xffffffffu, lane < ns && rms / (top + 1e-20) < tol);
     const int at = hit ? __ffs(hit) - 1 : ns - 1;
     *mx_out = __shfl_sync(0xffffffffu, mx, at < 0 ? 0 : at);
@@ -175,7 +169,8 @@ static __device__ __noinline__ int exit_rule(double own, double before, int ns, 
 // us per pass) is only evaluated when some sweep comes within a factor of the
 // tolerance; otherwise the smallest and the largest sum show that none meets
 // it.  Sums are not negative, so they order as their bits do.
-__device__ __forceinline__ void pass_done(LoopState &L, int e, const double *sq, int ns, int N, double tol)
+__device__ __forceinline__ void pass_done(LoopState &L, int e, const double *sq, int ns, int N, double tol,
+                                          double floor = -1e20)
 {
     const int lane = threadIdx.x & 31;
     const double own = sq[lane < ns ? lane : 0], before = L.inner_max_sq[e];
@@ -186,8 +181,9 @@ __device__ __forceinline__ void pass_done(LoopState &L, int e, const double *sq,
     const double least = __hiloint2double((int)nhi, 0);
     if (before > mx) mx = before;
     bool stop = false;
-    if (!(least > 1.001 * tol * tol * mx && least > 1e-30 * N && mhi < 0x7ff00000u))
-        stop = exit_rule(lane < ns ? own : 0.0, before, ns, N, tol, &mx) >= 0;
+    const double top = floor > 0.0 && floor * floor * N > mx ? floor * floor * N : mx;
+    if (!(least > 1.001 * tol * tol * top && least > 1e-30 * N && mhi < 0x7ff00000u))
+        stop = exit_rule(lane < ns ? own : 0.0, before, floor, ns, N, tol, &mx) >= 0;
     if (lane == 0) {
         L.inner_max_sq[e] = mx;
         L.sweeps[e] += ns;

@@ -75,3 +75,47 @@ def test_values_outside_the_reciprocal_range(gpu_ok, scale):
 @pytest.mark.parametrize("mu", [1e-20, 1e15])
 def test_diagonals_outside_the_reciprocal_range(gpu_ok, mu):
     check(dict(ifc.cavity2d(40, ny=36), dynamicViscosity=mu, density=1e-20 if mu < 1 else 1.0), 1)
+
+
+@pytest.mark.parametrize("prec", ["f", "d"])
+@pytest.mark.parametrize("nx,ny,sweeps,tol", [(64, 32, 23, 0.0), (65, 33, 7, 0.0), (109, 65, 60, 0.2), (24, 150, 40, 0.05)])
+def test_stored_coefficient_sweeps(gpu_ok, monkeypatch, nx, ny, sweeps, tol, prec):
+    """The temperature's sweeps in one launch (with the early exit in the middle
+    of them) against the per-pass launches: the same temperature and counts."""
+    cfg = dict(ifc.channel2d(nx, ny), precision=prec)
+    rng = np.random.default_rng(5)
+    state = {"uf": rng.uniform(-1e-3, 1e-3, (nx + 1) * ny), "vf": rng.uniform(-1e-3, 1e-3, nx * (ny + 1)),
+             "T": rng.uniform(280, 340, nx * ny)}
+    out = []
+    for off in ("0", "1"):
+        monkeypatch.setenv("IFC_PERSIST_OFF", off)
+        s = ifc.Solver(cfg)
+        for k, v in state.items():
+            s.set(k, v)
+        r = s.solve_energy(max_sweeps=sweeps, tol=tol)
+        out.append((r["sweeps"], r["converged"], s.get("T")))
+        s.close()
+    assert out[0][:2] == out[1][:2] and (tol == 0.0 or out[0][0] < sweeps), [o[:2] for o in out]
+    assert_bitwise(out[0][2], out[1][2], "T")
+
+
+@pytest.mark.parametrize("variant", ["1", "2"])
+@pytest.mark.parametrize("prec", ["f", "d"])
+def test_batch_regions(gpu_ok, monkeypatch, variant, prec):
+    """Batched cases of one region, one cell more, several regions per CTA and
+    different sweep counts of u and v, against the oracle over a fixed number of
+    outer iterations.  Tolerance: relative L2 1e-6 (every update is the oracle's;
+    only an inner exit decided on differently summed norms may move)."""
+    monkeypatch.setenv("IFC_BATCH_VARIANT", variant)
+    cases = [ifc.channel2d(64, 32), ifc.channel2d(65, 33), ifc.channel2d(3, 70), ifc.channel2d(230, 131)]
+    cases[1].update(nIter_u=3, nIter_v=11, nIter_p=7)
+    cases = [dict(c, precision=prec, numOuterIter=6, tol_u=1e-12, tol_v=1e-12, tol_p=1e-12) for c in cases]
+    res, fields, _ = ifc.batch_solve(cases)
+    for c, r, f in zip(cases, res, fields):
+        o = O.Oracle(to_oracle_cfg(dict(c, sweep_mode=O.GS_REDBLACK, check_every=r["sweeps_per_pass"])), prec)
+        n, _ = o.solve()
+        assert r["outer_iterations"] == n == 6
+        for k in ("u", "v", "p"):
+            a, b = f[k].astype(np.float64), o.field(k).astype(np.float64)
+            err = np.linalg.norm(a - b) / np.linalg.norm(b)
+            assert err < 1e-6, (c["nx"], c["ny"], k, err)

@@ -147,6 +147,9 @@ struct Engine : EngineBase {
     bool pc3d = false;
     PcBlocks pcb = {0, 0, 0, 0};
     size_t pc3d_smem = 0;
+    // The p' equation with its row links in shared memory (k_psolve3d), where they fit
+    static constexpr int kPsNT = sizeof(T) == 4 ? 768 : 512;
+    size_t ps3d_smem = 0;  // 0: they do not
     T *packed = nullptr;
     // The 3D momentum coefficients and sources of one solve, packed by the
     // first sweep (k_mom_half3d<T, true>): 10 values per slot
@@ -336,6 +339,7 @@ struct Engine : EngineBase {
     int prepare_pc3d()
     {
         pc3d = false;
+        ps3d_smem = 0;
         const char *off = std::getenv("IFC_PC3D_OFF");
         if (off && off[0] == '1') return IFC_OK;
         int dev = 0, optin = 0, coop = 0;
@@ -375,11 +379,32 @@ struct Engine : EngineBase {
         int per_sm = 0;
         IFC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kPcNT, smem));
         if (per_sm < 1 || (long long)per_sm * nsm < (long long)b.nbj * b.nbk) return IFC_OK;
-        int rc = alloc(&packed, (size_t)coop3d_slots(b, nx) * 8);
+        // k_psolve3d needs less (4 planes of padded slots and the exchanged
+        // rows) except in grids of one or two columns
+        const size_t pk_c = (size_t)coop3d_slots(b, nx) * 8;
+        const size_t pk_p = (size_t)b.nbj * b.nbk * b.bj * b.bk * 2 * psolve3d_half<T>(nx) * 5;
+        int rc = alloc(&packed, pk_c > pk_p ? pk_c : pk_p);
         if (rc != IFC_OK) return rc;
         pcb = b;
         pc3d_smem = smem;
         pc3d = true;
+        // The links between rows take 2.2 times the room of p' itself: up to
+        // about 140^3 in FP32 and 110^3 in FP64.  k_psolve3d gives a lane two
+        // cells of a row, so short rows leave its lanes idle: it is taken when a
+        // row fills 19 of 32 lanes.  p' solve, k_csolve3d against k_psolve3d, us:
+        // FP32 64^3 402 / 446, 80^3 626 / 483, 112^3 753 / 671, 128^3 849 / 740,
+        // 200x60x60 675 / 602, 20x300x300 1594 / 2671; FP64 64^3 464 / 484, 80^3
+        // 770 / 543, 97x89x101 991 / 697, 150x60x60 714 / 575, 20x200x200 1254 / 1758.
+        const int pairs = psolve3d_half<T>(nx) / 2;
+        if (pairs < 19 * ((pairs + 31) / 32)) return IFC_OK;
+        const size_t ps = psolve3d_smem_bytes<T>(b, nx);
+        auto kps = k_psolve3d<T, kPsNT>;
+        IFC_CK(cudaFuncGetAttributes(&fa, kps));
+        const int ps_max = optin - (int)fa.sharedSizeBytes;
+        if ((long long)ps > ps_max) return IFC_OK;
+        IFC_CK(cudaFuncSetAttribute(kps, cudaFuncAttributeMaxDynamicSharedMemorySize, ps_max));
+        IFC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kps, kPsNT, ps));
+        if (per_sm >= 1 && (long long)per_sm * nsm >= (long long)b.nbj * b.nbk) ps3d_smem = ps;
         return IFC_OK;
     }
 
@@ -387,11 +412,17 @@ struct Engine : EngineBase {
     // cooperative launch of n sweeps (k_csolve3d).
     void enq_csolve3d(const Params<T> &PP, CSys<T> sys, int n)
     {
+        launch_coop3d(k_csolve3d<T, kPcNT>, kPcNT, pc3d_smem, PP, f, ctl, partials, barrier, pcb, n, packed, sys);
+    }
+
+    template <typename... A, typename... U>
+    void launch_coop3d(void (*kern)(A...), int nt, size_t smem, U... args)
+    {
         cudaMemsetAsync(barrier, 0, sizeof(GridBarrier), stream);
         cudaLaunchConfig_t lc = {};
         lc.gridDim = dim3(pcb.nbj * pcb.nbk);
-        lc.blockDim = dim3(kPcNT);
-        lc.dynamicSmemBytes = pc3d_smem;
+        lc.blockDim = dim3(nt);
+        lc.dynamicSmemBytes = smem;
         lc.stream = stream;
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeCooperative;
@@ -400,12 +431,16 @@ struct Engine : EngineBase {
         lc.numAttrs = 1;
         const char *stall_env = std::getenv("IFC_TEST_STALL_BARRIER");  // failure-detection test, per launch
         const int stall = (stall_env && stall_env[0] == '1') ? 1 : 0;
-        cudaLaunchKernelEx(&lc, k_csolve3d<T, kPcNT>, PP, f, ctl, partials, barrier, pcb, n, packed, sys, stall);
+        cudaLaunchKernelEx(&lc, kern, args..., stall);
         ++launches;
     }
 
     void enq_pc_solve3d()
     {
+        if (ps3d_smem) {
+            launch_coop3d(k_psolve3d<T, kPsNT>, kPsNT, ps3d_smem, P, f, ctl, partials, barrier, pcb, cfg.n_iter_p, packed);
+            return;
+        }
         CSys<T> sys = {nullptr, f.sp, f.pc, EQ_P};
         enq_csolve3d(P, sys, cfg.n_iter_p);
     }

@@ -48,6 +48,27 @@ __device__ __forceinline__ unsigned int ld_acquire(const unsigned int *p)
     return v;
 }
 
+// The wait of a grid barrier: until `target` arrivals are in, or the limit.  One
+// L2 round trip per poll; the error flag and the clock are read every 64 polls
+// only, so they stay off the critical path.  A CTA that passes this barrier
+// while another gave up meets the flag at the next barrier, which the other
+// never reaches.
+__device__ __forceinline__ int await_arrivals(GridBarrier *b, unsigned int target)
+{
+    const unsigned long long t0 = global_ns();
+    unsigned int spins = 0;
+    while (ld_acquire(&b->count) < target) {
+        if ((++spins & 63u) == 0) {
+            if (*(volatile int *)&b->err) return 0;
+            if (global_ns() - t0 > kBarrierTimeoutNs) {
+                atomicExch(&b->err, 1);
+                return 0;
+            }
+        }
+    }
+    return 1;
+}
+
 // Grid barrier on a monotonically increasing arrival counter: each CTA adds
 // one arrival and waits until all G arrivals of this barrier are in, so the
 // critical path is one atomic plus the pollers' next read.  `epoch` counts
@@ -70,28 +91,36 @@ __device__ __forceinline__ bool grid_sync(GridBarrier *b, unsigned int nblocks, 
         // cycles for 108 CTAs, the polls then queue before the arrivals.)
         unsigned int old;
         asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(&b->count) : "memory");
-        if (old + 1 < target) {
-            // One L2 round trip per poll; the error flag and the clock are
-            // read every 64 polls only, so they stay off the critical path.
-            // A CTA that passes this barrier while another gave up meets the
-            // flag at the next barrier, which the other never reaches.
-            const unsigned long long t0 = global_ns();
-            unsigned int spins = 0;
-            while (ld_acquire(&b->count) < target) {
-                if ((++spins & 63u) == 0) {
-                    if (*(volatile int *)&b->err) { good = 0; break; }
-                    if (global_ns() - t0 > kBarrierTimeoutNs) {
-                        atomicExch(&b->err, 1);
-                        good = 0;
-                        break;
-                    }
-                }
-            }
-        }
+        if (old + 1 < target) good = await_arrivals(b, target);
         ok = good;
     }
     __syncthreads();
     return ok != 0;
+}
+
+// The two halves of grid_sync, with work of the CTA's own between them that no
+// other CTA reads before a later barrier.  Every thread of a CTA of NT threads
+// calls both.
+template <int NT>
+__device__ __forceinline__ void grid_arrive(GridBarrier *b, unsigned int nblocks, unsigned int &epoch)
+{
+    if (nblocks == 1) return;
+    ++epoch;
+    if (threadIdx.x < 32) {
+        asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
+        if (threadIdx.x == 0)
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&b->count) : "memory");
+    } else {
+        asm volatile("bar.arrive 1, %0;" ::"n"(NT) : "memory");
+    }
+}
+
+__device__ __forceinline__ bool grid_wait(GridBarrier *b, unsigned int nblocks, unsigned int epoch)
+{
+    __shared__ int ok;
+    if (nblocks > 1 && threadIdx.x == 0) ok = await_arrivals(b, epoch * nblocks);
+    __syncthreads();
+    return nblocks == 1 || ok != 0;
 }
 
 // Sum column r of partials (one value per CTA) for r < ncol in a fixed order;

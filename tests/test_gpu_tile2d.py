@@ -99,6 +99,30 @@ def test_stored_coefficient_sweeps(gpu_ok, monkeypatch, nx, ny, sweeps, tol, pre
     assert_bitwise(out[0][2], out[1][2], "T")
 
 
+@pytest.mark.parametrize("prec", ["f", "d"])
+@pytest.mark.parametrize("nx,ny,nz,bc", [(73, 12, 11, "cavity"), (77, 31, 30, "cavity"), (80, 3, 3, "cavity"), (128, 13, 14, "channel"),
+                                         (151, 20, 9, "channel"), (154, 3, 40, "cavity")])
+def test_3d_pressure_rows(gpu_ok, monkeypatch, nx, ny, nz, bc, prec):
+    """The 3D p' solve with its row links in shared memory, at odd and even rows,
+    one and two warps of cells per row, blocks of a single row, with the early
+    exit in the middle, against the per-half-sweep kernels: the same p' and
+    sweep count.  Tolerance: exact (the same updates in the same order)."""
+    base = ifc.cavity3d(16) if bc == "cavity" else ifc.channel2d(16, 16)
+    cfg = dict(base, dim=3, nx=nx, ny=ny, nz=nz, precision=prec, nIter_w=base["nIter_u"])
+    for tol in (0.0, 0.3):
+        out = []
+        for off in ("0", "1"):
+            monkeypatch.setenv("IFC_PC3D_OFF", off)
+            s = ifc.Solver(dict(cfg, tol_p=tol, nIter_p=9))
+            for k, v in seeded_state(cfg, 4, s.dtype).items():
+                s.set(k, v)
+            s.iterate(2)
+            out.append([s.get(k) for k in ("pc", "p", "u", "v", "w", "uf")])
+            s.close()
+        for k, a, b in zip(("pc", "p", "u", "v", "w", "uf"), *out):
+            assert_bitwise(a, b, f"tol {tol} {k}")
+
+
 @pytest.mark.parametrize("variant", ["1", "2"])
 @pytest.mark.parametrize("prec", ["f", "d"])
 def test_batch_regions(gpu_ok, monkeypatch, variant, prec):

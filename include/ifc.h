@@ -214,9 +214,10 @@ typedef struct ifc_batch_result {
  * iteration as ifc_solve.  A case's size class (up to 64^2, 160^2, larger
  * cells) selects how its sweeps run: whole-row sweeps, or temporally blocked
  * passes of a tile shape and sweeps per pass; the first batch of a process
- * that meets a class times every variant on copies of the class's median case
- * and keeps the fastest for the rest of the process (IFC_BATCH_VARIANT=<k> in
- * the environment forces variant k).  results: n
+ * that meets a class times every variant on copies of the class's median case,
+ * and every batch takes the variant with which its own cases of the class would
+ * be finished first (IFC_BATCH_VARIANT=<k> in the environment forces variant
+ * k).  results: n
  * entries.  fields_out (optional): n host pointers, each receiving u, v, p of
  * its case (3*nx*ny values of the case's precision), or NULL entries.
  * device_ms (optional): device time of the whole batch.  Device memory is

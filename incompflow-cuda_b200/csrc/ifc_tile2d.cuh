@@ -77,26 +77,27 @@ __device__ __forceinline__ double quot_div(double n, double y)
     return q;
 }
 
-// n / y outside the range of the reciprocal.  A tiny quotient that is still
-// normal is formed scaled up (both scalings are exact), which keeps the
-// division on its fast path; fronts of a flow that develops from rest pass
-// through these magnitudes.
-template <typename T>
-__device__ __forceinline__ T quot_rare(T n, T y)
-{
-    using K = KnownDiv<T>;
-    if (abs_t(n) < K::small) {
-        const T q = quot_div(n * K::up, y) * K::down;
-        if (abs_t(q) >= K::tiny) return q;
-    }
-    return quot_div(n, y);
-}
-
 // Whether divisor y may be used with a precomputed reciprocal.
 template <typename T>
 __device__ __forceinline__ bool divisor_ok(T y)
 {
     return abs_t(y) >= KnownDiv<T>::ylo && abs_t(y) <= KnownDiv<T>::yhi;
+}
+
+// n / y outside the range of the reciprocal.  A tiny quotient that is still
+// normal is formed scaled up (both scalings are exact), which keeps the
+// division on its fast path; fronts of a flow that develops from rest pass
+// through these magnitudes.  Only for a divisor in the ordinary range: divided
+// by a smaller one the scaled numerator overflows although n / y does not.
+template <typename T>
+__device__ __forceinline__ T quot_rare(T n, T y)
+{
+    using K = KnownDiv<T>;
+    if (abs_t(n) < K::small && divisor_ok(y)) {
+        const T q = quot_div(n * K::up, y) * K::down;
+        if (abs_t(q) >= K::tiny) return q;
+    }
+    return quot_div(n, y);
 }
 
 __device__ __forceinline__ float fma1(float a, float b, float c) { return __fmaf_rn(a, b, c); }

@@ -511,8 +511,8 @@ __global__ void __launch_bounds__(NT, 1) k_psolve3d(const __grid_constant__ Para
                     const Pair<T> qv = fma2(fma2(q0, y, np), pair(z), q0);
                     T v0 = qv.lo(), v1 = qv.hi();
                     if (max(range_key(v0), range_key(v1)) > KnownDiv<T>::kSpan) {
-                        if (range_key(v0) > KnownDiv<T>::kSpan && (np.lo() != (T)0 || z.x != z.x)) v0 = quot_rare(np.lo(), -y.lo());
-                        if (range_key(v1) > KnownDiv<T>::kSpan && (np.hi() != (T)0 || z.y != z.y)) v1 = quot_rare(np.hi(), -y.hi());
+                        if (range_key(v0) > KnownDiv<T>::kSpan && (np.lo() != (T)0 || z.x != z.x)) v0 = quot_far(np.lo(), -y.lo(), z.x);
+                        if (range_key(v1) > KnownDiv<T>::kSpan && (np.hi() != (T)0 || z.y != z.y)) v1 = quot_far(np.hi(), -y.hi(), z.y);
                     }
                     const T d0 = relax * (v0 - c.x);
                     T d1 = relax * (v1 - c.y);

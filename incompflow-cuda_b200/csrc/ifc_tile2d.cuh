@@ -27,8 +27,9 @@
 // System/6000 processor", IBM J. Res. Dev. 34, 1990; N. Brisebarre, J.-M.
 // Muller, S. K. Raina, "Accelerating correctly rounded floating-point division
 // when the divisor is known in advance", IEEE Trans. Comput. 53, 2004), away
-// from overflow and underflow.  Quotients outside a safe range (zero among
-// them), and cells whose diagonal is outside one, take the division itself.
+// from overflow and underflow.  Tiny quotients are formed scaled up; those near
+// overflow, and cells whose diagonal is outside the range of the reciprocal, take
+// the division itself.
 #pragma once
 
 #include "ifc_kernels.cuh"
@@ -44,12 +45,14 @@ template <typename T>
 struct KnownDiv;
 template <>
 struct KnownDiv<float> {
-    static constexpr float ylo = 0x1p-40f, yhi = 0x1p40f, up = 0x1p64f, down = 0x1p-64f, tiny = 0x1p-126f, small = 0x1p-20f;
+    static constexpr float ylo = 0x1p-40f, yhi = 0x1p40f, small = 0x1p-20f, large = 0x1p120f;
+    static constexpr float up = 0x1p64f, down = 0x1p-64f, tiny = 0x1p-126f, ulp = 0x1p-149f, half = 0x1p-86f;
     static constexpr unsigned kLow = (127u - 62u) << 24, kSpan = (124u << 24) - 1u;
 };
 template <>
 struct KnownDiv<double> {
-    static constexpr double ylo = 0x1p-200, yhi = 0x1p200, up = 0x1p400, down = 0x1p-400, tiny = 0x1p-1022, small = 0x1p-500;
+    static constexpr double ylo = 0x1p-200, yhi = 0x1p200, small = 0x1p-500, large = 0x1p1000;
+    static constexpr double up = 0x1p400, down = 0x1p-400, tiny = 0x1p-1022, ulp = 0x1p-1074, half = 0x1p-675;
     static constexpr unsigned kLow = (1023u - 700u) << 21, kSpan = (1400u << 21) - 1u;
 };
 
@@ -84,24 +87,50 @@ __device__ __forceinline__ bool divisor_ok(T y)
     return abs_t(y) >= KnownDiv<T>::ylo && abs_t(y) <= KnownDiv<T>::yhi;
 }
 
-// n / y outside the range of the reciprocal.  A tiny quotient that is still
-// normal is formed scaled up (both scalings are exact), which keeps the
-// division on its fast path; fronts of a flow that develops from rest pass
-// through these magnitudes.  Only for a divisor in the ordinary range: divided
-// by a smaller one the scaled numerator overflows although n / y does not.
-template <typename T>
-__device__ __forceinline__ T quot_rare(T n, T y)
-{
-    using K = KnownDiv<T>;
-    if (abs_t(n) < K::small && divisor_ok(y)) {
-        const T q = quot_div(n * K::up, y) * K::down;
-        if (abs_t(q) >= K::tiny) return q;
-    }
-    return quot_div(n, y);
-}
-
 __device__ __forceinline__ float fma1(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma1(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+// The quotient of n < small, given q = RN(m / y) of the numerator scaled up, m =
+// up * n (exact): q scaled back.  That rounds a second time when the result is
+// subnormal (or the smallest normal number, which can come from below): where q
+// lies halfway between two subnormals -- `half` is half their distance, scaled
+// up -- the sign of the exact residual tells on which side the quotient is.
+template <typename T>
+__device__ __forceinline__ T scaled_back(T q, T m, T y)
+{
+    using K = KnownDiv<T>;
+    T d = q * K::down;
+    if (abs_t(d) <= K::tiny) {
+        const T diff = q - d * K::up, r = fma1(-q, y, m);
+        if (abs_t(diff) == K::half && r != (T)0 && (diff > (T)0) == ((r > (T)0) == (y > (T)0)))
+            d += diff > (T)0 ? K::ulp : -K::ulp;
+    }
+    return d;
+}
+
+// n / y for a divisor in [ylo, yhi] and z = RN(1/y), whatever the magnitude of
+// n; `ok` tells whether it is (not where the quotient comes near overflow, nor
+// where y or z is out of range or not a number).
+template <typename T>
+__device__ __forceinline__ T quot_scaled(T n, T y, T z, bool &ok)
+{
+    using K = KnownDiv<T>;
+    const bool low = abs_t(n) < K::small;
+    const T m = n * (low ? K::up : (T)1);
+    T q = m * z;
+    q = fma1(fma1(-q, y, m), z, q);
+    ok = abs_t(q) <= K::large && divisor_ok(y);
+    return low ? scaled_back(q, m, y) : q;
+}
+
+// The same in every case, out of line.
+template <typename T>
+static __device__ __noinline__ T quot_far(T n, T y, T z)
+{
+    bool ok;
+    const T q = quot_scaled(n, y, z, ok);
+    return ok ? q : quot_div(n, y);
+}
 
 // n / y given z = RN(1/y).
 template <typename T>
@@ -110,7 +139,7 @@ __device__ __forceinline__ T quot_known(T n, T y, T z)
     T q = n * z;
     q = fma1(fma1(-q, y, n), z, q);
     if (range_key(q) > KnownDiv<T>::kSpan || !divisor_ok(y)) {
-        if (n != (T)0 || !divisor_ok(y)) q = quot_rare(n, y);
+        if (n != (T)0 || !divisor_ok(y)) q = quot_far(n, y, z);
     }
     return q;
 }
@@ -311,6 +340,68 @@ struct Links {
     }
 };
 
+// The quotients q = n / diagonal whose bit in `todo` is set (bit 2*J*f + 2*j + h),
+// which lie outside the range of half_sweep's formula.  Fronts of a flow that
+// develops from rest pass through all small magnitudes, down to zero, many warps
+// at a time, and every CTA waits for the slowest: 1024x256 channel from rest,
+// us per iteration over the first 20, with a division each (twice for subnormal
+// quotients) 290 FP32 / 523 FP64, this way 138 / 428.  FP32 takes all values at
+// once, scaled up where they are small; in FP64 that costs registers that the
+// sweeps need (developed flow 308 -> 319), so one value at a time.
+template <typename RT, typename T, int COLOR, int F>
+__device__ __forceinline__ void far_quotients(const Links<RT, T> &a, const T (&n)[F][RT::R / 2][2],
+                                              T (&q)[F][RT::R / 2][2], unsigned todo, bool force)
+{
+    using K = KnownDiv<T>;
+    constexpr int J = RT::R / 2;
+    constexpr bool at_once = sizeof(T) == 4;
+    if (at_once && !force) {
+        todo = 0;  // what is left: quotients near overflow
+#pragma unroll
+        for (int f = 0; f < F; ++f)
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+                const Pair<T> z = a.Z.pair(COLOR, j), c = a.C.pair(COLOR, j);
+                const bool low0 = abs_t(n[f][j][0]) < K::small, low1 = abs_t(n[f][j][1]) < K::small;
+                const Pair<T> m = mul2(Pair<T>(n[f][j][0], n[f][j][1]), Pair<T>(low0 ? K::up : (T)1, low1 ? K::up : (T)1));
+                Pair<T> w = mul2(m, z);
+                w = fma2(fma2(w, c, m), z, w);
+                if (!(abs_t(w.lo()) <= K::large)) todo |= 1u << (2 * J * f + 2 * j);
+                if (!(abs_t(w.hi()) <= K::large)) todo |= 2u << (2 * J * f + 2 * j);
+                q[f][j][0] = low0 ? scaled_back(w.lo(), m.lo(), -c.lo()) : w.lo();
+                q[f][j][1] = low1 ? scaled_back(w.hi(), m.hi(), -c.hi()) : w.hi();
+            }
+        if (!todo) return;
+    }
+    // In loops, so that they take little code.
+    T tn[F * 2 * J], ty[2 * J];
+#pragma unroll
+    for (int i = 0; i < 2 * J; ++i) {
+        ty[i] = -a.C.v[COLOR][i >> 1][i & 1];
+#pragma unroll
+        for (int f = 0; f < F; ++f) tn[2 * J * f + i] = n[f][i >> 1][i & 1];
+    }
+    if (at_once) {
+#pragma unroll 1
+        for (int i = 0; i < F * 2 * J; ++i)
+            if (todo >> i & 1u) tn[i] = quot_div(tn[i], ty[i % (2 * J)]);
+    } else {
+#pragma unroll 1
+        for (unsigned rest = todo; rest; rest &= rest - 1) {
+            const int i = __ffs(rest) - 1;
+            const T y = ty[i % (2 * J)];
+            const bool low = abs_t(tn[i]) < K::small && divisor_ok(y);
+            const T m = low ? tn[i] * K::up : tn[i], w = quot_div(m, y);
+            tn[i] = low ? scaled_back(w, m, y) : w;
+        }
+    }
+#pragma unroll
+    for (int f = 0; f < F; ++f)
+#pragma unroll
+        for (int i = 0; i < 2 * J; ++i)
+            if (todo >> (2 * J * f + i) & 1u) q[f][i >> 1][i & 1] = tn[2 * J * f + i];
+}
+
 // One half sweep of colour COLOR over the lane's rows for the F unknowns x[f]
 // (one, or u and v with their common links: twice the independent work for
 // the latency of one).  With SUM, acc[f][k] receives the squared changes of
@@ -363,8 +454,7 @@ __device__ __forceinline__ void half_sweep(Cells<T, RT::R> *const (&xs)[F], cons
         }
     }
     if (force || key > KnownDiv<T>::kSpan) {
-        // Rare: the divisions themselves, in a loop so that they take little
-        // code.  A zero numerator needs none: its quotient is a zero already
+        // A zero numerator needs nothing more: its quotient is a zero already
         // (only the sign may differ, which q - x and x + d erase).
         unsigned todo = 0;
 #pragma unroll
@@ -373,25 +463,7 @@ __device__ __forceinline__ void half_sweep(Cells<T, RT::R> *const (&xs)[F], cons
             for (int i = 0; i < 2 * J; ++i)
                 if (force || (range_key(q[f][i >> 1][i & 1]) > KnownDiv<T>::kSpan && n[f][i >> 1][i & 1] != (T)0))
                     todo |= 1u << (2 * J * f + i);
-        if (todo) {
-            T tn[F * 2 * J], ty[2 * J];
-#pragma unroll
-            for (int i = 0; i < 2 * J; ++i) {
-                ty[i] = -a.C.v[COLOR][i >> 1][i & 1];
-#pragma unroll
-                for (int f = 0; f < F; ++f) tn[2 * J * f + i] = n[f][i >> 1][i & 1];
-            }
-#pragma unroll 1
-            for (unsigned rest = todo; rest; rest &= rest - 1) {
-                const int i = __ffs(rest) - 1;
-                tn[i] = quot_rare(tn[i], ty[i % (2 * J)]);
-            }
-#pragma unroll
-            for (int f = 0; f < F; ++f)
-#pragma unroll
-                for (int i = 0; i < 2 * J; ++i)
-                    if (todo >> (2 * J * f + i) & 1u) q[f][i >> 1][i & 1] = tn[2 * J * f + i];
-        }
+        if (todo) far_quotients<RT, T, COLOR, F>(a, n, q, todo, force);
     }
 #pragma unroll
     for (int f = 0; f < F; ++f) {

@@ -51,3 +51,40 @@ def test_3d_pressure_rows(gpu_ok, monkeypatch, prec, mu, rho, scale):
     for k, a, b in zip(("pc", "p", "u", "v", "w", "uf"), *out):
         assert np.isfinite(b).all(), k
         assert_bitwise(a, b, k)
+
+
+@pytest.mark.parametrize("prec,scale", [("f", 1e-30), ("f", 1e-36), ("f", 2e-38), ("f", 1e-41), ("d", 1e-306),
+                                        ("d", 3e-308), ("d", 1e-312)])
+def test_small_and_subnormal_quotients(gpu_ok, prec, scale):
+    """Ordinary diagonals under numerators whose quotients are near the smallest
+    normal number or below it."""
+    cfg = still(ifc.cavity2d(70, ny=40), precision=prec)
+    o = O.Oracle(to_oracle_cfg(cfg), prec)
+    s = ifc.Solver(cfg)
+    load_both(o, s, {k: (v * scale).astype(s.dtype) for k, v in seeded_state(cfg, 5, np.float64).items()})
+    for it in range(2):
+        s.iterate(1)
+        o.outer_iteration()
+        o.bc_face_vel()
+        for k in ("u", "v", "p", "uf", "vf"):
+            assert_bitwise(s.get(k), o.field(k), f"it{it} {k}")
+
+
+@pytest.mark.parametrize("prec,iters", [("f", 3), ("d", 9)])
+def test_front_from_rest(gpu_ok, prec, iters):
+    """A channel flow developing from rest: the front of u, v and p' passes
+    through every magnitude down to zero (FP32: 1e-45, FP64: 1e-324)."""
+    cfg = dict(ifc.channel2d(900, 40), precision=prec)
+    o = O.Oracle(to_oracle_cfg(cfg), prec)
+    o.init_face_vel()
+    o.bc_face_vel()
+    s = ifc.Solver(cfg)
+    for it in range(iters):
+        s.iterate(1)
+        o.outer_iteration()
+        o.bc_face_vel()
+        for k in ("u", "v", "p", "uf", "vf"):
+            assert_bitwise(s.get(k), o.field(k), f"it{it} {k}")
+    u = abs(o.field("u"))
+    tiny = np.finfo(u.dtype).tiny
+    assert (u == 0).any() and ((u > 0) & (u < tiny)).any()

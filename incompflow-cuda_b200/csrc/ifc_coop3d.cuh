@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(NT, 1) k_csolve3d(Params<T> P, Fields<T> f, Ct
                 for (int w = 0; w < NT / 32; ++w) t += red[w];
                 partials[(size_t)(2 * (s & 1) + color) * G + blockIdx.x] = t;
             }
-            if (!grid_sync(bar, G, epoch)) {
+            if (!grid_sync<false>(bar, G, epoch)) {
                 failed = true;
                 break;
             }

@@ -682,6 +682,8 @@ __global__ void __launch_bounds__(32 * NW_, 1) k_simple2d(const __grid_constant_
 
         T *const pcc = bp(pcur);  // the current p'
         if (npass_p == 0) {       // no p' sweeps: p' = 0 (src/Solver.cu:193)
+            // no p' pass takes a decision left over from the momentum passes
+            if (pending.kind) resolve_now();
 #pragma unroll 1
             for (int t = blockIdx.x; t < ntiles; t += G) {
                 const TileBox tl = tile_box(pa.tiles, t, nx, ny);

@@ -143,3 +143,23 @@ def test_batch_regions(gpu_ok, monkeypatch, variant, prec):
             a, b = f[k].astype(np.float64), o.field(k).astype(np.float64)
             err = np.linalg.norm(a - b) / np.linalg.norm(b)
             assert err < 1e-6, (c["nx"], c["ny"], k, err)
+
+
+@pytest.mark.parametrize("nu,nv,tu,tv", [(15, 10, 2.0, 0.0), (10, 15, 0.0, 2.0), (15, 10, 0.0, 0.0), (5, 5, 2.0, 2.0)])
+def test_sweep_counts_without_pressure_sweeps(gpu_ok, monkeypatch, nu, nv, tu, tv):
+    """nIter_p = 0 with one component's sweeps ended early and the other's in an
+    earlier pass than the last: the counts of the per-pass launches, and the
+    same fields."""
+    cfg = dict(ifc.channel2d(97, 70), nIter_u=nu, nIter_v=nv, nIter_p=0, tol_u=tu, tol_v=tv)
+    out = []
+    for off in ("0", "1"):
+        monkeypatch.setenv("IFC_PERSIST_OFF", off)
+        s = ifc.Solver(cfg)
+        for k, v in seeded_state(cfg, 6, s.dtype).items():
+            s.set(k, v)
+        r = s.iterate(1)
+        out.append((list(r["sweeps"]), r["cell_updates"], [s.get(k) for k in ("u", "v", "p", "uf", "vf")]))
+        s.close()
+    assert out[0][:2] == out[1][:2], [o[:2] for o in out]
+    for a, b in zip(out[0][2], out[1][2]):
+        assert_bitwise(a, b)

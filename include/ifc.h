@@ -110,7 +110,7 @@ typedef struct ifc_config {
     int linear_solver;                /* IFC_GAUSS_SEIDEL (default) or IFC_JACOBI */
     int criterion;                    /* IFC_CRIT_PER_FIELD (default), _REFERENCE or _RESIDUAL */
     int pin_pressure;                 /* -1 auto (closed domains), 0 off, 1 on */
-    int sweeps_per_pass;              /* sweeps fused per device pass; 0 = tuned default */
+    int sweeps_per_pass;              /* sweeps between the inner early-exit checks, fused in one or two device passes; 0 = tuned default */
     int log_level;                    /* 0 silent, 1 reference log cadence on stdout */
     const double *inlet_profile;      /* optional west-face inlet velocity per boundary cell (ny*nz) */
     void *stream;                     /* cudaStream_t to run on, or NULL for a private stream */

@@ -144,6 +144,7 @@ __global__ void __launch_bounds__(32 * NW_, 1)
     const double floor = ctl->inner_max[eq];
     if (tid == 0) {
         L.stop[eq] = ctl->stop[eq];
+        L.hit[eq] = 0;
         L.sweeps[eq] = 0;
         L.cell_updates[eq] = 0;
         L.inner_max_sq[eq] = -1.0;
@@ -185,7 +186,7 @@ __global__ void __launch_bounds__(32 * NW_, 1)
     pending.kind = kPendNone;
     auto take = [&]() {  // by warp 0, after a block barrier
         if (warp != 0) return;
-        pass_done(L, eq, tot, pending.n0, N, g.tol[eq], floor);
+        pass_done(L, eq, tot, pending.n0, N, g.tol[eq], true, floor);
         if (tid == 0) last_sq = tot[pending.n0 - 1];
     };
 #pragma unroll 1

@@ -178,11 +178,13 @@ template <>
 struct RegionShapes<float> {
     static constexpr int n = 3;
     static constexpr RegionShape s[n] = {{2, 12, 0.85}, {2, 16, 1.0}, {4, 16, 1.6}};
+    static constexpr double alone = 0.3;  // what a pass gains without grid barriers
 };
 template <>
 struct RegionShapes<double> {
     static constexpr int n = 3;
     static constexpr RegionShape s[n] = {{2, 12, 0.8}, {2, 16, 1.0}, {2, 18, 1.1}};
+    static constexpr double alone = 0.3;
 };
 
 template <typename T, int I>
@@ -215,7 +217,7 @@ static int persist_kernel(Engine<T> &e, bool launch, int *capacity)
             cudaFuncGetAttributes(&fa, kern) != cudaSuccess)
             return IFC_CUDA_ERROR;
         const int dyn_max = optin - (int)fa.sharedSizeBytes;
-        if ((long long)smem > dyn_max) return IFC_UNSUPPORTED;  // deep passes of the largest region
+        if ((long long)smem > dyn_max) return IFC_UNSUPPORTED;
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn_max) != cudaSuccess)
             return IFC_CUDA_ERROR;
         int per_sm = 0;
@@ -234,13 +236,13 @@ static int persist_kernel(Engine<T> &e, bool launch, int *capacity)
                : IFC_CUDA_ERROR;
 }
 
-template <typename T>
+template <typename T, int I = 0>
 static int persist_dispatch(Engine<T> &e, int shape, bool launch, int *capacity)
 {
-    constexpr int n = RegionShapes<T>::n;
-    if (shape == n - 1) return persist_kernel<T, n - 1>(e, launch, capacity);
-    if (shape == n - 2) return persist_kernel<T, n - 2>(e, launch, capacity);
-    return persist_kernel<T, 0>(e, launch, capacity);
+    if constexpr (I + 1 < RegionShapes<T>::n) {
+        if (shape > I) return persist_dispatch<T, I + 1>(e, shape, launch, capacity);
+    }
+    return persist_kernel<T, I>(e, launch, capacity);
 }
 
 static inline int persist_ks(int want)
@@ -273,35 +275,51 @@ int Engine<T>::prepare_persist()
     pa.n_iter[2] = 0;
     pa.n_iter[3] = cfg.n_iter_p;
     pa.pin = pin ? 1 : 0;
-    pa.ks = persist_ks(spp_persist);
     pa.stall_test = 0;
     int cap_env = 0;
     if (const char *cap = std::getenv("IFC_PERSIST_MAX_CTAS")) cap_env = std::atoi(cap);
+    // Passes of six and more sweeps need halos of 24 and more cells, which leave
+    // little of a region (FP64 500x190, 8 sweeps: 433 us per outer iteration).  They
+    // may be split into two each; the early exit is then checked after every
+    // second pass, so the values are the same (same example: 103 us).
+    const int check = persist_ks(spp_persist);
+    const int n_m = cfg.n_iter_u > cfg.n_iter_v ? cfg.n_iter_u : cfg.n_iter_v;
     double best = 0.0;
-    for (int s = 0; s < RegionShapes<T>::n; ++s) {
-        const RegionShape &sh = RegionShapes<T>::s[s];
-        TileGrid tg;
-        tg.H = 2 * pa.ks;
-        if (!split_axis(P.g.nx, 64, tg.H, &tg.kx, &tg.Ix) || !split_axis(P.g.ny, sh.R * sh.NW, tg.H, &tg.ky, &tg.Iy))
-            continue;
-        int capacity = 0;
-        if (persist_dispatch<T>(*this, s, false, &capacity) != IFC_OK) {
-            cudaGetLastError();
-            continue;
+    int best_ks = check;
+    for (int group = 1; group <= (check >= 6 && check % 2 == 0 ? 2 : 1); ++group)
+        for (int s = 0; s < RegionShapes<T>::n; ++s) {
+            const RegionShape &sh = RegionShapes<T>::s[s];
+            pa.ks = check / group;
+            TileGrid tg;
+            tg.H = 2 * pa.ks;
+            if (!split_axis(P.g.nx, 64, tg.H, &tg.kx, &tg.Ix) || !split_axis(P.g.ny, sh.R * sh.NW, tg.H, &tg.ky, &tg.Iy))
+                continue;
+            int capacity = 0;
+            if (persist_dispatch<T>(*this, s, false, &capacity) != IFC_OK) {
+                cudaGetLastError();
+                continue;
+            }
+            if (cap_env > 0 && capacity > cap_env) capacity = cap_env;
+            if (capacity < 1) continue;
+            const long long tiles = (long long)tg.kx * tg.ky;
+            const long long per = (tiles + capacity - 1) / capacity;
+            // Passes of an outer iteration times the cost of one: half of a
+            // pass of five sweeps is its sweeps, half what comes with every
+            // pass (64x64 FP32: 66 us per iteration with 3 sweeps, 50 with 5).
+            const int passes = (n_m + pa.ks - 1) / pa.ks + (cfg.n_iter_p + pa.ks - 1) / pa.ks;
+            // (a single tile runs without grid barriers)
+            const double cost = (passes > 0 ? passes : 1) * (0.5 + 0.1 * pa.ks) *
+                                ((double)per * sh.cost - (tiles == 1 ? RegionShapes<T>::alone : 0.0));
+            if (persist && cost >= best) continue;
+            best = cost;
+            best_ks = pa.ks;
+            persist = true;
+            persist_shape = s;
+            persist_grid = (int)((tiles + per - 1) / per);
+            pa.tiles = tg;
+            pa.group = group;
         }
-        if (cap_env > 0 && capacity > cap_env) capacity = cap_env;
-        if (capacity < 1) continue;
-        const long long tiles = (long long)tg.kx * tg.ky;
-        const long long per = (tiles + capacity - 1) / capacity;
-        // (a single tile runs without grid barriers)
-        const double cost = (double)per * sh.cost - (tiles == 1 ? 0.3 : 0.0);
-        if (persist && cost >= best) continue;
-        best = cost;
-        persist = true;
-        persist_shape = s;
-        persist_grid = (int)((tiles + per - 1) / per);
-        pa.tiles = tg;
-    }
+    pa.ks = best_ks;
     return IFC_OK;
 }
 
@@ -341,13 +359,13 @@ static cudaError_t coef_kernel(Engine<T> &e, CoefCall<T> *call, int *capacity)
     return cudaLaunchCooperativeKernel((const void *)kern, dim3(tg.kx * tg.ky), dim3(RT::NT), args, smem, e.stream);
 }
 
-template <typename T>
+template <typename T, int I = 0>
 static cudaError_t coef_dispatch(Engine<T> &e, int shape, CoefCall<T> *call, int *capacity)
 {
-    constexpr int n = RegionShapes<T>::n;
-    if (shape == n - 1) return coef_kernel<T, n - 1>(e, call, capacity);
-    if (shape == n - 2) return coef_kernel<T, n - 2>(e, call, capacity);
-    return coef_kernel<T, 0>(e, call, capacity);
+    if constexpr (I + 1 < RegionShapes<T>::n) {
+        if (shape > I) return coef_dispatch<T, I + 1>(e, shape, call, capacity);
+    }
+    return coef_kernel<T, I>(e, call, capacity);
 }
 
 template <typename T>
@@ -368,7 +386,7 @@ bool Engine<T>::coef_coop()
         if (!split_axis(P.g.nx, 64, tg.H, &tg.kx, &tg.Ix) || !split_axis(P.g.ny, sh.R * sh.NW, tg.H, &tg.ky, &tg.Iy))
             continue;
         const long long tiles = (long long)tg.kx * tg.ky;
-        const double cost = sh.cost - (tiles == 1 ? 0.3 : 0.0);
+        const double cost = sh.cost - (tiles == 1 ? RegionShapes<T>::alone : 0.0);
         int capacity = 0;
         if (coef_dispatch<T>(*this, s, nullptr, &capacity) != cudaSuccess) {
             cudaGetLastError();

@@ -157,6 +157,7 @@ constexpr int kMassColumn = 2 * kSetColumns;
 struct LoopState {
     int it, it_begin, it_stop, act, log_level, log_n, status, done;
     int stop[4], sweeps[4];
+    int hit[4];                 // the early-exit rule was met (it ends the sweeps where a group of passes ends)
     long long cell_updates[4];  // by equation, so that two warps can count at once
     double inner_max_sq[4];     // largest sum of squared changes of a sweep; negative: none yet
     double maxn[8];
@@ -166,6 +167,7 @@ struct PersistArgs {
     int n_iter[4];
     int pin;
     int ks;          // sweeps per pass
+    int group;       // passes per early-exit check: the sweeps end early after a multiple of ks * group only
     TileGrid tiles;  // tiles for a halo of 2*ks cells
     int stall_test;  // failure-detection test: CTA 0 leaves before its first barrier
 };
@@ -201,8 +203,9 @@ static __device__ __noinline__ int exit_rule(double own, double before, double f
 // us per pass) is only evaluated when some sweep comes within a factor of the
 // tolerance; otherwise the smallest and the largest sum show that none meets
 // it.  Sums are not negative, so they order as their bits do.
+// ends: the pass ends a group, so the sweeps may end here.
 __device__ __forceinline__ void pass_done(LoopState &L, int e, const double *sq, int ns, int N, double tol,
-                                          double floor = -1e20)
+                                          bool ends, double floor = -1e20)
 {
     const int lane = threadIdx.x & 31;
     const double own = sq[lane < ns ? lane : 0], before = L.inner_max_sq[e];
@@ -220,13 +223,14 @@ __device__ __forceinline__ void pass_done(LoopState &L, int e, const double *sq,
         L.inner_max_sq[e] = mx;
         L.sweeps[e] += ns;
         L.cell_updates[e] += (long long)ns * N;
-        if (stop) L.stop[e] = 1;
+        if (stop) L.hit[e] = 1;
+        if (ends && L.hit[e]) L.stop[e] = 1;
     }
 }
 
-// Bookkeeping of the last pass of a phase: its sums could only set an
-// early-exit flag for passes that do not follow (the flags are reset with
-// every outer iteration), so they are not reduced.
+// Bookkeeping of the passes of a phase's last group: their sums could only set
+// an early-exit flag for passes that do not follow (the flags are reset with
+// every outer iteration), so they are not taken.
 __device__ __forceinline__ void pass_count(LoopState &L, int e, int ns, int N)
 {
     L.sweeps[e] += ns;
@@ -289,6 +293,7 @@ static __device__ __noinline__ void finish_norms(const Geo<T> &g, LoopState &L, 
     if (lane < 8) L.maxn[lane] = mq;
     if (lane < 4) {
         L.stop[lane] = 0;
+        L.hit[lane] = 0;
         L.sweeps[lane] = 0;
         L.inner_max_sq[lane] = -1.0;
     }
@@ -321,8 +326,10 @@ enum { kPendNone = 0, kPendMomentum, kPendP, kPendNorms };
 struct Pending {
     int kind, ncol, n0, n1;
     int part;  // offset of the first column in the partials
-    __device__ __forceinline__ void set(int k, int p, int columns, int a, int b)
+    bool ends; // the pass ends a group
+    __device__ __forceinline__ void set(int k, int p, int columns, int a, int b, bool e = true)
     {
+        ends = e;
         kind = k;
         ncol = columns;
         n0 = a;
@@ -373,7 +380,7 @@ __device__ __forceinline__ void decide(const Geo<T> &g, LoopState &L, Ctl *ctl, 
     }
     const int e = warp == 1 ? EQ_V : pd.kind == kPendP ? EQ_P : EQ_U;
     const int n = warp == 1 ? pd.n1 : pd.n0;
-    if (n > 0) pass_done(L, e, tot + (warp == 1 ? ks : 0), n, g.N, g.tol[e]);
+    if (n > 0) pass_done(L, e, tot + (warp == 1 ? ks : 0), n, g.N, g.tol[e], pd.ends);
 }
 
 // Faces whose loads one thread has in flight in the Rhie-Chow phase, and cells
@@ -416,6 +423,7 @@ __global__ void __launch_bounds__(32 * NW_, 1) k_simple2d(const __grid_constant_
         for (int q = 0; q < 4; ++q) {
             L.cell_updates[q] = 0;
             L.stop[q] = 0;
+            L.hit[q] = 0;
             L.sweeps[q] = 0;
             L.inner_max_sq[q] = -1.0;
         }
@@ -426,6 +434,9 @@ __global__ void __launch_bounds__(32 * NW_, 1) k_simple2d(const __grid_constant_
 
     const int npass_m = (max(pa.n_iter[0], pa.n_iter[1]) + ks - 1) / ks;
     const int npass_p = (pa.n_iter[3] + ks - 1) / ks;
+    // the first pass of a phase's last group
+    const int tail_m = npass_m > 0 ? (npass_m - 1) / pa.group * pa.group : 0;
+    const int tail_p = npass_p > 0 ? (npass_p - 1) / pa.group * pa.group : 0;
     bool failed = false;
     unsigned int epoch = 0;
     int set = 0;
@@ -494,8 +505,7 @@ __global__ void __launch_bounds__(32 * NW_, 1) k_simple2d(const __grid_constant_
                 const bool au = ns0 > 0 && (pass == 0 || !L.stop[EQ_U]);
                 const bool av = ns1 > 0 && (pass == 0 || !L.stop[EQ_V]);
                 if (!au && !av && pass > 0) break;
-                // The sums of a phase's last pass are never reduced.
-                const bool last = pass >= npass_m - 1;
+                const bool sums = pass < tail_m;
                 const bool keep = one && pass > 0;
                 bool cu = au, cv = av;  // whether this pass's u, v count
 #pragma unroll 1
@@ -516,7 +526,7 @@ __global__ void __launch_bounds__(32 * NW_, 1) k_simple2d(const __grid_constant_
                     if (pending.kind)
                         decide<T>(g, L, ctl, tot, tot_mass, pending, ks);
                     sweeps2<RT, T>(u, v, a, pl, g.relax[EQ_U], g.relax[EQ_V], force, au ? ns0 : 0,
-                                   av ? ns1 : 0, ks, !last, t != (int)blockIdx.x, sred);
+                                   av ? ns1 : 0, ks, sums, t != (int)blockIdx.x, sred);
                     if (pending.kind) {
                         if (ns0 == 0 && ns1 == 0) __syncthreads();  // (the sweeps have barriers otherwise)
                         pending.kind = kPendNone;
@@ -536,16 +546,16 @@ __global__ void __launch_bounds__(32 * NW_, 1) k_simple2d(const __grid_constant_
                 }
                 if (L.done || (pass > 0 && !cu && !cv)) break;
                 mcur ^= 1;
-                if (!last) column_partials<NT>(sred, 2 * ks, partials + set * set_len, G, tot);
+                if (sums) column_partials<NT>(sred, 2 * ks, partials + set * set_len, G, tot);
                 if (!grid_sync(bar, G, epoch)) { failed = true; break; }
-                if (last) {
+                if (!sums) {
                     if (tid == 0) {
                         if (cu) pass_count(L, EQ_U, ns0, N);
                         if (cv) pass_count(L, EQ_V, ns1, N);
                     }
-                    break;
+                    continue;
                 }
-                pending.set(kPendMomentum, set * set_len, 2 * ks, cu ? ns0 : 0, cv ? ns1 : 0);
+                pending.set(kPendMomentum, set * set_len, 2 * ks, cu ? ns0 : 0, cv ? ns1 : 0, (pass + 1) % pa.group == 0);
                 set ^= 1;
                 if (!one) resolve_now();
             }
@@ -643,7 +653,7 @@ __global__ void __launch_bounds__(32 * NW_, 1) k_simple2d(const __grid_constant_
             for (int pass = 0; pass < npass_p; ++pass) {
                 const int ns = clamp_sweeps(pa.n_iter[3], pass, ks);
                 if (pass > 0 && L.stop[EQ_P]) break;
-                const bool last = pass == npass_p - 1;
+                const bool sums = pass < tail_p;
                 const bool keep = one && pass > 0;
                 bool stopped = false;
 #pragma unroll 1
@@ -657,7 +667,7 @@ __global__ void __launch_bounds__(32 * NW_, 1) k_simple2d(const __grid_constant_
                     __syncthreads();
                     if (pending.kind)
                         decide<T>(g, L, ctl, tot, tot_mass, pending, ks);
-                    sweeps1<RT, T>(x, a, pl, g.relax[EQ_P], force, ns, ks, !last, t != (int)blockIdx.x, sred);
+                    sweeps1<RT, T>(x, a, pl, g.relax[EQ_P], force, ns, ks, sums, t != (int)blockIdx.x, sred);
                     if (pending.kind) {
                         pending.kind = kPendNone;
                         stopped = L.stop[EQ_P] != 0;
@@ -667,13 +677,13 @@ __global__ void __launch_bounds__(32 * NW_, 1) k_simple2d(const __grid_constant_
                 }
                 if (stopped) break;
                 pcur ^= 1;
-                if (!last) column_partials<NT>(sred, ks, partials + set * set_len, G, tot);
+                if (sums) column_partials<NT>(sred, ks, partials + set * set_len, G, tot);
                 if (!grid_sync(bar, G, epoch)) { failed = true; break; }
-                if (last) {
+                if (!sums) {
                     if (tid == 0) pass_count(L, EQ_P, ns, N);
-                    break;
+                    continue;
                 }
-                pending.set(kPendP, set * set_len, ks, ns, 0);
+                pending.set(kPendP, set * set_len, ks, ns, 0, (pass + 1) % pa.group == 0);
                 set ^= 1;
                 if (!one) resolve_now();
             }

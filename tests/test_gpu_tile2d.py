@@ -163,3 +163,28 @@ def test_sweep_counts_without_pressure_sweeps(gpu_ok, monkeypatch, nu, nv, tu, t
     assert out[0][:2] == out[1][:2], [o[:2] for o in out]
     for a, b in zip(out[0][2], out[1][2]):
         assert_bitwise(a, b)
+
+
+@pytest.mark.parametrize("prec", ["f", "d"])
+@pytest.mark.parametrize("spp,every,nx,ny,cap", [(6, 6, 97, 70, 0), (7, 6, 150, 101, 2), (8, 8, 64, 64, 0), (8, 8, 150, 101, 2),
+                                                 (9, 8, 33, 31, 0), (10, 10, 97, 70, 0), (16, 10, 300, 37, 3)])
+@pytest.mark.parametrize("tol", [0.0, 0.3])
+def test_deep_passes(gpu_ok, monkeypatch, prec, spp, every, nx, ny, cap, tol):
+    """Six to sixteen sweeps per pass: one launch, and the early exit taken after
+    every 6, 8 or 10 sweeps, whatever the passes are split into.  Tolerance: exact."""
+    if cap:
+        monkeypatch.setenv("IFC_PERSIST_MAX_CTAS", str(cap))
+    cfg = dict(ifc.channel2d(nx, ny), precision=prec, sweeps_per_pass=spp, nIter_u=17, nIter_v=9, nIter_p=23, tol_u=tol,
+               tol_v=tol / 3, tol_p=2 * tol)
+    o = O.Oracle(dict(to_oracle_cfg(cfg), check_every=every), prec)
+    s = ifc.Solver(cfg)
+    load_both(o, s, seeded_state(cfg, 8, s.dtype))
+    for it in range(2):
+        r = s.iterate(1)
+        assert r["kernel_launches"] == 3, r
+        want = o.outer_iteration()["sweeps"]
+        o.bc_face_vel()
+        assert list(r["sweeps"]) == list(want), (it, r["sweeps"], want)
+        for k in ("u", "v", "p", "uf", "vf"):
+            assert_bitwise(s.get(k), o.field(k), f"it{it} {k}")
+    s.close()

@@ -167,7 +167,12 @@ namespace ifc {
 // the larger regions waste less on halos and win once they save a round
 // (1024x256: 112 us with 64 rows; 32 rows would take 4 rounds).  FP64 has half
 // the registers per cell: 64 rows do not fit, 36 rows (500x190 in one round)
-// do.
+// do; its half sweeps take in proportion to their rows (64x64, us per outer
+// iteration with 24, 28, 32 and 36 rows: 67, 76, 85, 106), so a single tile gains
+// little from having no barriers (33x31: 79 us in one of 32 rows, 65 in three of
+// 24), 20 rows serve passes of up to four sweeps (33x31, 4 sweeps: 88 -> 70) and
+// 28 rows tall grids that 24 do not hold in one round (29x621: 83 -> 77; FP32 56
+// -> 54).
 struct RegionShape {
     int R, NW;
     double cost;
@@ -176,15 +181,15 @@ template <typename T>
 struct RegionShapes;
 template <>
 struct RegionShapes<float> {
-    static constexpr int n = 3;
-    static constexpr RegionShape s[n] = {{2, 12, 0.85}, {2, 16, 1.0}, {4, 16, 1.6}};
+    static constexpr int n = 4;
+    static constexpr RegionShape s[n] = {{2, 12, 0.85}, {2, 14, 0.92}, {2, 16, 1.0}, {4, 16, 1.6}};
     static constexpr double alone = 0.3;  // what a pass gains without grid barriers
 };
 template <>
 struct RegionShapes<double> {
-    static constexpr int n = 3;
-    static constexpr RegionShape s[n] = {{2, 12, 0.8}, {2, 16, 1.0}, {2, 18, 1.1}};
-    static constexpr double alone = 0.3;
+    static constexpr int n = 5;
+    static constexpr RegionShape s[n] = {{2, 10, 0.7}, {2, 12, 0.8}, {2, 14, 0.9}, {2, 16, 1.0}, {2, 18, 1.2}};
+    static constexpr double alone = 0.1;
 };
 
 template <typename T, int I>

@@ -188,3 +188,11 @@ def test_deep_passes(gpu_ok, monkeypatch, prec, spp, every, nx, ny, cap, tol):
         for k in ("u", "v", "p", "uf", "vf"):
             assert_bitwise(s.get(k), o.field(k), f"it{it} {k}")
     s.close()
+
+
+@pytest.mark.parametrize("prec", ["f", "d"])
+@pytest.mark.parametrize("nx,ny,spp", [(33, 31, 5), (64, 20, 4), (65, 21, 4), (40, 23, 2), (29, 621, 5), (64, 28, 5), (70, 29, 5)])
+def test_small_and_narrow_regions(gpu_ok, nx, ny, spp, prec):
+    """Regions of 20 and 28 rows: filled exactly, one row more, and the tall
+    narrow grid that takes them at the default depth."""
+    check(dict(ifc.channel2d(nx, ny), precision=prec, sweeps_per_pass=spp), 2)

@@ -510,9 +510,9 @@ __global__ void __launch_bounds__(NT, 1) k_psolve3d(const __grid_constant__ Para
                     const Pair<T> q0(np.lo() * z.x, np.hi() * z.y);
                     const Pair<T> qv = fma2(fma2(q0, y, np), pair(z), q0);
                     T v0 = qv.lo(), v1 = qv.hi();
-                    if (max(range_key(v0), range_key(v1)) > KnownDiv<T>::kSpan) {
-                        if (range_key(v0) > KnownDiv<T>::kSpan && (np.lo() != (T)0 || z.x != z.x)) v0 = quot_far(np.lo(), -y.lo(), z.x);
-                        if (range_key(v1) > KnownDiv<T>::kSpan && (np.hi() != (T)0 || z.y != z.y)) v1 = quot_far(np.hi(), -y.hi(), z.y);
+                    if (max(quot_key(v0), quot_key(v1)) > KnownDiv<T>::kSpanQ) {
+                        if (quot_key(v0) > KnownDiv<T>::kSpanQ && (np.lo() != (T)0 || z.x != z.x)) v0 = quot_far(np.lo(), -y.lo(), z.x);
+                        if (quot_key(v1) > KnownDiv<T>::kSpanQ && (np.hi() != (T)0 || z.y != z.y)) v1 = quot_far(np.hi(), -y.hi(), z.y);
                     }
                     const T d0 = relax * (v0 - c.x);
                     T d1 = relax * (v1 - c.y);

@@ -36,30 +36,50 @@
 
 namespace ifc {
 
-// Ranges in which the corrected quotient is exact: |y| in [ylo, yhi] and |q| in
-// [2^-62, 2^62) (FP64: [2^-700, 2^700)) keep the residual n - q y (a multiple
-// of ulp(q) ulp(y)) and every intermediate normal.  range_key(q) maps |q| to an
-// unsigned number that is at most kSpan inside the range and larger for any
-// other value, zero, infinity and NaN among them.
+// Ranges in which the corrected quotient is exact: |y| in [ylo, yhi] and |n| in
+// [2^-85, 2^80) (FP64: [2^-820, 2^800)) keep the residual n - q y (a multiple of
+// ulp(q) ulp(y), at least 2^-47 |n|) and every intermediate normal.
+// range_key(n) maps |n| to an unsigned number that is at most kSpan inside the
+// range and larger for any other value, zero, infinity and NaN among them.
+// Where z may be no number, quot_key looks at the quotient instead: |q| in
+// [2^-62, 2^62) (FP64: [2^-700, 2^700)) does as well, for every y in its range.
 template <typename T>
 struct KnownDiv;
 template <>
 struct KnownDiv<float> {
     static constexpr float ylo = 0x1p-40f, yhi = 0x1p40f, small = 0x1p-20f, large = 0x1p120f;
     static constexpr float up = 0x1p64f, down = 0x1p-64f, tiny = 0x1p-126f, ulp = 0x1p-149f, half = 0x1p-86f;
-    static constexpr unsigned kLow = (127u - 62u) << 24, kSpan = (124u << 24) - 1u;
+    static constexpr unsigned kLow = (127u - 85u) << 24, kSpan = (165u << 24) - 1u;
+    static constexpr unsigned kLowQ = (127u - 62u) << 24, kSpanQ = (124u << 24) - 1u;
 };
 template <>
 struct KnownDiv<double> {
     static constexpr double ylo = 0x1p-200, yhi = 0x1p200, small = 0x1p-500, large = 0x1p1000;
     static constexpr double up = 0x1p400, down = 0x1p-400, tiny = 0x1p-1022, ulp = 0x1p-1074, half = 0x1p-675;
-    static constexpr unsigned kLow = (1023u - 700u) << 21, kSpan = (1400u << 21) - 1u;
+    static constexpr unsigned kLow = (1023u - 820u) << 21, kSpan = (1620u << 21) - 1u;
+    static constexpr unsigned kLowQ = (1023u - 700u) << 21, kSpanQ = (1400u << 21) - 1u;
 };
 
-__device__ __forceinline__ unsigned range_key(float q) { return __float_as_uint(q) * 2u - KnownDiv<float>::kLow; }
-__device__ __forceinline__ unsigned range_key(double q)
+__device__ __forceinline__ unsigned magnitude(float a) { return __float_as_uint(a) * 2u; }
+__device__ __forceinline__ unsigned magnitude(double a) { return (unsigned)__double2hiint(a) * 2u; }
+template <typename T>
+__device__ __forceinline__ unsigned range_key(T n)
 {
-    return (unsigned)__double2hiint(q) * 2u - KnownDiv<double>::kLow;
+    return magnitude(n) - KnownDiv<T>::kLow;
+}
+template <typename T>
+__device__ __forceinline__ unsigned quot_key(T q)
+{
+    return magnitude(q) - KnownDiv<T>::kLowQ;
+}
+// Which of the two the sweeps look at: the numerator's range is wider (29x621
+// channel, whose core holds tiny values for long, 69 -> 64 us per outer
+// iteration), but with four rows per lane it costs registers (developed 2048x512
+// 426 -> 436 us).
+template <int R, typename T>
+__device__ __forceinline__ unsigned far_key(T n, T q)
+{
+    return R == 2 ? range_key(n) : quot_key(q);
 }
 __device__ __forceinline__ float abs_t(float a) { return fabsf(a); }
 __device__ __forceinline__ double abs_t(double a) { return fabs(a); }
@@ -138,7 +158,7 @@ __device__ __forceinline__ T quot_known(T n, T y, T z)
 {
     T q = n * z;
     q = fma1(fma1(-q, y, n), z, q);
-    if (range_key(q) > KnownDiv<T>::kSpan || !divisor_ok(y)) {
+    if (range_key(n) > KnownDiv<T>::kSpan || !divisor_ok(y)) {
         if (n != (T)0 || !divisor_ok(y)) q = quot_far(n, y, z);
     }
     return q;
@@ -413,6 +433,7 @@ __device__ __forceinline__ void half_sweep(Cells<T, RT::R> *const (&xs)[F], cons
                                            double (&acc)[F][2])
 {
     constexpr int J = RT::R / 2, OC = 1 - COLOR;
+    constexpr unsigned span = RT::R == 2 ? KnownDiv<T>::kSpan : KnownDiv<T>::kSpanQ;
     const Pair<T> minus(-(T)1, -(T)1);
     T n[F][J][2], q[F][J][2];
     T below[F], above[F];
@@ -450,10 +471,10 @@ __device__ __forceinline__ void half_sweep(Cells<T, RT::R> *const (&xs)[F], cons
             n[f][j][1] = num.hi();
             q[f][j][0] = quo.lo();
             q[f][j][1] = quo.hi();
-            key = max(key, max(range_key(q[f][j][0]), range_key(q[f][j][1])));
+            key = max(key, max(far_key<RT::R>(n[f][j][0], q[f][j][0]), far_key<RT::R>(n[f][j][1], q[f][j][1])));
         }
     }
-    if (force || key > KnownDiv<T>::kSpan) {
+    if (force || key > span) {
         // A zero numerator needs nothing more: its quotient is a zero already
         // (only the sign may differ, which q - x and x + d erase).
         unsigned todo = 0;
@@ -461,7 +482,7 @@ __device__ __forceinline__ void half_sweep(Cells<T, RT::R> *const (&xs)[F], cons
         for (int f = 0; f < F; ++f)
 #pragma unroll
             for (int i = 0; i < 2 * J; ++i)
-                if (force || (range_key(q[f][i >> 1][i & 1]) > KnownDiv<T>::kSpan && n[f][i >> 1][i & 1] != (T)0))
+                if (force || (far_key<RT::R>(n[f][i >> 1][i & 1], q[f][i >> 1][i & 1]) > span && n[f][i >> 1][i & 1] != (T)0))
                     todo |= 1u << (2 * J * f + i);
         if (todo) far_quotients<RT, T, COLOR, F>(a, n, q, todo, force);
     }

@@ -214,11 +214,15 @@ typedef struct ifc_batch_result {
  * iteration as ifc_solve.  A case's size class (up to 64^2, 160^2, larger
  * cells) selects how its sweeps run: whole-row sweeps, or temporally blocked
  * passes of a tile shape and sweeps per pass; the first batch of a process
- * that meets a class times every variant on copies of the class's median case,
- * and every batch takes the variant with which its own cases of the class would
- * be finished first (IFC_BATCH_VARIANT=<k> in the environment forces variant
- * k).  results: n
- * entries.  fields_out (optional): n host pointers, each receiving u, v, p of
+ * that meets a class times every variant on copies of the class's median case.
+ * Every batch then takes the variants with which it would be finished first
+ * (IFC_BATCH_VARIANT=<k> in the environment forces variant k), which changes no
+ * value: the inner early exit of a case is checked after every
+ * result.sweeps_per_pass sweeps -- those of the class's variant of highest
+ * throughput, kept for the process (IFC_BATCH_CHECK=<n> forces n, in every
+ * process) -- whichever variant runs it.  (Variants add their FP64 sums in
+ * different orders: norms may differ in the last bits, and with them the p'
+ * mean that is taken out of closed FP64 cases.)  results: n entries.  fields_out (optional): n host pointers, each receiving u, v, p of
  * its case (3*nx*ny values of the case's precision), or NULL entries.
  * device_ms (optional): device time of the whole batch.  Device memory is
  * allocated for the call and freed before it returns.  No counterpart in the

@@ -1,7 +1,7 @@
 // ifc_batch.cu -- many independent 2D SIMPLE solves in one persistent kernel.
 //
-// Work distribution: the kernel is launched as thread-block clusters of kCL
-// CTAs; each cluster takes the next case from a device queue (cases are queued
+// Work distribution: the kernel is launched as thread-block clusters (of kCL
+// CTAs; of two in variant 1, below); each cluster takes the next case from a device queue (cases are queued
 // largest first), runs up to `chunk` SIMPLE outer iterations of it
 // (src/Solver.cu:160-289, the same per-cell arithmetic as every other path,
 // ifc_physics.cuh), saves its loop state and takes the next case.  The CTAs of
@@ -41,6 +41,7 @@ struct BCase {
     Params<T> P;
     long long off_c, off_uf, off_vf;  // offsets into the pools
     int n_iter[4];
+    int check;  // sweeps between the inner early-exit checks
     int pin;
     int max_outer;
 };
@@ -68,10 +69,24 @@ struct BQueue {
 
 // Case-local loop state shared by the threads of one CTA.
 struct CaseLoop {
-    int stop[4];
+    int limit[4];  // sweeps of this inner solve: n_iter, or where the early exit ends it
+    int hit[4];    // the early-exit rule was met
     double inner_max[4];
     int sweeps[4];
 };
+
+// The early-exit rule of src/Solver.cu:955-962 on the sum of squared changes of
+// sweep s (from 0) of equation e.  Once met it ends the inner solve after the
+// next multiple of `check` sweeps.
+__device__ __forceinline__ void inner_rule(CaseLoop &L, int e, double sq, int s, int n, int check, int N, double tol)
+{
+    const double rms = sqrt(sq / (double)N);
+    if (rms > L.inner_max[e]) L.inner_max[e] = rms;
+    if (rms / (L.inner_max[e] + 1e-20) < tol) {
+        L.hit[e] = 1;
+        L.limit[e] = min(n, (s / check + 1) * check);
+    }
+}
 
 // Sum NV values over the threads of the CTA into this CTA's slot `part`
 // (shared memory); call with every thread.
@@ -198,7 +213,8 @@ __global__ void __cluster_dims__(kCL, 1, 1) __launch_bounds__(kBNT, 4)
         for (int k = 0; k < chunk && !S.done; ++k) {
             if (tid == 0)
                 for (int e = 0; e < 4; ++e) {
-                    L.stop[e] = 0;
+                    L.limit[e] = C.n_iter[e];
+                    L.hit[e] = 0;
                     L.inner_max[e] = -1e20;
                     L.sweeps[e] = 0;
                 }
@@ -221,8 +237,8 @@ __global__ void __cluster_dims__(kCL, 1, 1) __launch_bounds__(kBNT, 4)
             // ---- momentum sweeps, coefficients on the fly (kernels.cuh:97-334, 926-1005)
             const int nm = max(C.n_iter[0], C.n_iter[1]);
             for (int s = 0; s < (nm > 0 ? nm : 1); ++s) {
-                const bool du = s < C.n_iter[0] && !L.stop[EQ_U];
-                const bool dv = s < C.n_iter[1] && !L.stop[EQ_V];
+                const bool du = s < L.limit[EQ_U];
+                const bool dv = s < L.limit[EQ_V];
                 if (!du && !dv && s > 0) break;
                 double sq[2] = {0.0, 0.0};
                 for (int color = 0; color < 2; ++color) {
@@ -264,9 +280,7 @@ __global__ void __cluster_dims__(kCL, 1, 1) __launch_bounds__(kBNT, 4)
                 if (tid == 0) {
                     for (int m = 0; m < 2; ++m) {
                         if (!(m == 0 ? du : dv)) continue;
-                        const double rms = sqrt(tot[m] / (double)N);
-                        if (rms > L.inner_max[m]) L.inner_max[m] = rms;
-                        if (rms / (L.inner_max[m] + 1e-20) < g.tol[m]) L.stop[m] = 1;
+                        if (!L.hit[m]) inner_rule(L, m, tot[m], s, C.n_iter[m], C.check, N, g.tol[m]);
                         L.sweeps[m]++;
                     }
                 }
@@ -317,7 +331,7 @@ __global__ void __cluster_dims__(kCL, 1, 1) __launch_bounds__(kBNT, 4)
             // ---- p' sweeps from p' = 0 (src/Solver.cu:193-196, kernels.cuh:502-540)
             const double mass_sq = tot[8];
             for (int s = 0; s < C.n_iter[3]; ++s) {
-                if (L.stop[EQ_P]) break;
+                if (s >= L.limit[EQ_P]) break;
                 double sq[1] = {0.0};
                 for (int color = 0; color < 2; ++color) {
                     const int zm = s == 0 ? (color == 0 ? 1 : 2) : 0;
@@ -347,9 +361,7 @@ __global__ void __cluster_dims__(kCL, 1, 1) __launch_bounds__(kBNT, 4)
                 }
                 cluster_total<1>(cl, &part[s & 1][2], tot);
                 if (tid == 0) {
-                    const double rms = sqrt(tot[0] / (double)N);
-                    if (rms > L.inner_max[EQ_P]) L.inner_max[EQ_P] = rms;
-                    if (rms / (L.inner_max[EQ_P] + 1e-20) < g.tol[EQ_P]) L.stop[EQ_P] = 1;
+                    if (!L.hit[EQ_P]) inner_rule(L, EQ_P, tot[0], s, C.n_iter[EQ_P], C.check, N, g.tol[EQ_P]);
                     L.sweeps[EQ_P]++;
                 }
                 __syncthreads();
@@ -489,9 +501,10 @@ __global__ void __cluster_dims__(kCL, 1, 1) __launch_bounds__(kBNT, 4)
 // for the smallest cases (two CTAs each, one or two tiles), variant 2 for the
 // larger ones.  The autotuner times every variant on copies of a size class's
 // median case (a fixed number of outer iterations) the first time the class is
-// met in a process; from these times a batch chooses, per class, the variant
-// whose cases would be finished first (choose_variant).  IFC_BATCH_VARIANT=<k>
-// forces variant k.
+// met in a process; from these times a batch chooses the variants with which it
+// would be finished first (choose_variants).  IFC_BATCH_VARIANT=<k> forces
+// variant k.  The variants compute the same values: the interval of the inner
+// early-exit checks belongs to the class (Tuned::check), not to the variant.
 constexpr int kNumVariants = 3;
 constexpr int kVariantSweeps[kNumVariants] = {1, 3, 5};
 constexpr int kNumClasses = 3;
@@ -592,83 +605,175 @@ static void launch_variant(int v, int nclusters, cudaStream_t st, const BCase<T>
         }                                                                          \
     } while (0)
 
+// How a case is solved: its variant and the sweeps between its inner early-exit
+// checks.  The second decides the values, the first only how soon they are there.
+struct Plan {
+    int variant = 0, check = 1;
+};
+
 template <typename T>
-static int batch_run(const ifc_config *cfgs, int n, const std::vector<int> &wanted, ifc_batch_result *res,
-                     void *const *fields_out,
-                     double *ms_out);
+static int batch_run(const ifc_config *cfgs, int n, const std::vector<Plan> &plan, ifc_batch_result *res,
+                     void *const *fields_out, double *ms_out);
 
 // What the autotuner measured for each size class and precision in this process.
 struct Tuned {
     bool done = false;
-    double cells = 0;             // of the probed case
-    double lat[kNumVariants];     // time of the probe's iterations on one cluster of a busy GPU (0: failed)
-    int clusters[kNumVariants];   // clusters that run at once
+    int check = 1;               // of the variant with the highest throughput
+    int nx = 0, ny = 0;          // of the probed case
+    double lone[kNumVariants];   // time of the probe's iterations with one cluster running (0: failed)
+    double full[kNumVariants];   // with every cluster running
+    int clusters[kNumVariants];  // clusters that run at once
 };
 static std::mutex g_tune_mu;
 static Tuned g_tuned[2][kNumClasses];
 
-// The variant that finishes cases of the given cells (one size class) first:
-// each goes, largest first, to the cluster that is free first, and takes the
-// probed time scaled by its cells.  Many cases go to the variant with the
-// highest throughput (whole rows: 71 small clusters), few to the one that
-// finishes the largest case soonest (a case has one cluster: 48 uneven cavities
-// 90 ms with whole rows, the 256x256 one alone takes that long, 67 ms with
-// regions in registers).
-static int choose_variant(const Tuned &t, std::vector<double> cells)
+// One class's cases of a batch, for choose_variants.
+struct ClassWork {
+    Tuned t;
+    std::vector<std::pair<int, int>> grids;  // nx, ny
+};
+
+// Rounds of a cluster over a case in variant v, to which the time of a case is
+// about proportional: chunks of 32 cells of a colour per warp (whole rows), or
+// tiles per CTA; and what stands for the barriers (64x64 against 96x32: 0.75 of
+// the time with whole rows, 1 chunk against 2; 1.45 in variant 1, 2 rounds against 1).
+template <typename T>
+static double rounds(int v, int nx, int ny)
 {
-    std::sort(cells.begin(), cells.end(), [](double a, double b) { return a > b; });
-    int best = 0;
-    double best_end = 0.0;
-    for (int v = 0; v < kNumVariants; ++v) {
-        if (t.lat[v] <= 0.0 || t.clusters[v] < 1) continue;
-        std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
-        for (int k = 0; k < t.clusters[v]; ++k) free_at.push(0.0);
-        double end = 0.0;
-        for (double c : cells) {
-            const double e = free_at.top() + t.lat[v] * c / t.cells;
-            free_at.pop();
-            free_at.push(e);
-            end = std::max(end, e);
-        }
-        if (best_end == 0.0 || end < best_end) {
-            best_end = end;
-            best = v;
+    if (v == 0) {
+        const int warps = kCL * kBNT / 32;
+        return 2.0 + ((ny + warps - 1) / warps) * (((nx + 1) / 2 + 31) / 32);
+    }
+    const VariantLaunch vl = variant_launch<T>(v);
+    TileGrid g;
+    g.H = 2 * kVariantSweeps[v];
+    split_axis(nx, vl.tx, g.H, &g.kx, &g.Ix);
+    split_axis(ny, vl.ty, g.H, &g.ky, &g.Iy);
+    return 1.1 + (g.kx * g.ky + vl.cl - 1) / vl.cl;
+}
+
+// Estimated time of one queue: the cases of the classes that take variant v, each
+// to the cluster that is free first, largest first.  A cluster runs slower the
+// more of them run (between the two probed times).
+template <typename T>
+static double queue_time(const std::vector<ClassWork> &cw, const std::vector<int> &choice, int v)
+{
+    std::vector<double> work;  // times on a lone cluster
+    double sum = 0.0, busy = 0.0;
+    int clusters = 0;
+    for (size_t k = 0; k < cw.size(); ++k) {
+        if (choice[k] != v) continue;
+        const Tuned &t = cw[k].t;
+        clusters = t.clusters[v];
+        const double round = t.lone[v] / rounds<T>(v, t.nx, t.ny);
+        for (const auto &g : cw[k].grids) {
+            work.push_back(round * rounds<T>(v, g.first, g.second));
+            sum += work.back();
+            busy += work.back() * (t.full[v] / t.lone[v]);
         }
     }
-    return best;
+    if (work.empty()) return 0.0;
+    std::sort(work.begin(), work.end(), [](double a, double b) { return a > b; });
+    const double slow = busy / sum;  // slowdown with every cluster running
+    // All running cases slow down alike, so they finish in the order of their
+    // `clock` (lone time passed); real time follows the number running.
+    std::priority_queue<double, std::vector<double>, std::greater<double>> ends;
+    double clock = 0.0, now = 0.0;
+    size_t next = 0;
+    while (next < work.size() || !ends.empty()) {
+        while (next < work.size() && (int)ends.size() < clusters) ends.push(clock + work[next++]);
+        const double m = (double)ends.size();
+        const double step = ends.top() - clock;
+        now += step * (1.0 + (slow - 1.0) * (clusters > 1 ? (m - 1.0) / (clusters - 1.0) : 0.0));
+        clock = ends.top();
+        ends.pop();
+    }
+    return now;
+}
+
+// The variants with which the batch as a whole would be finished first: the
+// queues of different variants run one after the other, so the classes are
+// decided together.  (Each class by itself: 96 uneven cavities 143 ms with two
+// queues that each wait for their last case, 111 ms with one.)  Many cases go
+// to the variant with the highest throughput (whole rows: 71 small clusters),
+// few to the one that finishes the largest case soonest (a case has one
+// cluster: 48 uneven cavities 102 ms with whole rows, 67 ms with regions in
+// registers).
+template <typename T>
+static std::vector<int> choose_variants(const std::vector<ClassWork> &cw)
+{
+    const std::vector<int> first(cw.size(), 0);
+    std::vector<int> choice = first, best = first;
+    double best_time = 0.0;
+    for (;;) {
+        bool valid = true;
+        for (size_t k = 0; k < cw.size(); ++k)
+            valid = valid && cw[k].t.lone[choice[k]] > 0.0 && cw[k].t.clusters[choice[k]] > 0;
+        if (valid) {
+            double t = 0.0;
+            for (int v = 0; v < kNumVariants; ++v) t += queue_time<T>(cw, choice, v);
+            // the estimates are good to about 5 %: whole rows for all, the first
+            // choice looked at, unless others are faster by that
+            if (best_time == 0.0 || t < (best == first ? 0.95 : 1.0) * best_time) {
+                best_time = t;
+                best = choice;
+            }
+            if (getenv("IFC_VERBOSE")) {
+                fprintf(stderr, "ifc_batch variants");
+                for (int c : choice) fprintf(stderr, " %d", c);
+                fprintf(stderr, ": %.3f ms estimated\n", t);
+            }
+        }
+        size_t k = 0;
+        while (k < choice.size() && ++choice[k] == kNumVariants) choice[k++] = 0;
+        if (k == choice.size()) return best;
+    }
 }
 
 template <typename T>
 static Tuned autotune(int cls, const ifc_config &rep)
 {
-    // Probe: copies of the class's median case, 20 outer iterations each (no
-    // early stop), enough copies to fill the GPU with any variant.
-    constexpr int kCopies = 96;
-    std::vector<ifc_config> probe(kCopies, rep);
-    for (ifc_config &c : probe) {
-        c.convection_scheme = IFC_CONV_UPWIND;  // the variants differ in their sweeps only
-        c.tol_u = c.tol_v = c.tol_w = c.tol_p = 0.0;
-        c.tol_mass = 0.0;
-        c.num_outer_iter = 20;
-    }
-    std::vector<ifc_batch_result> r(kCopies);
+    // Probe: the class's median case, 20 outer iterations (no early stop), alone
+    // and as many copies as a variant runs at once.
     Tuned t;
-    t.done = true;
-    t.cells = (double)rep.nx * rep.ny;
+    t.nx = rep.nx;
+    t.ny = rep.ny;
+    double best = 0.0;
     for (int v = 0; v < kNumVariants; ++v) {
-        double ms = 0.0;
-        t.lat[v] = 0.0;
+        t.lone[v] = t.full[v] = 0.0;
         t.clusters[v] = 0;
-        if (variant_clusters<T>(v, &t.clusters[v]) != cudaSuccess) {
+        if (variant_clusters<T>(v, &t.clusters[v]) != cudaSuccess || t.clusters[v] < 1) {
             cudaGetLastError();
             continue;
         }
-        const std::vector<int> forced(kCopies, v);
-        if (batch_run<T>(probe.data(), kCopies, forced, r.data(), nullptr, &ms) != IFC_OK) continue;
-        const int at_once = std::max(1, std::min(kCopies, t.clusters[v]));
-        t.lat[v] = ms / ((kCopies + at_once - 1) / at_once);
+        double ms[2] = {0.0, 0.0};
+        bool ok = true;
+        for (int q = 0; q < 2; ++q) {
+            const int copies = q == 0 ? 1 : t.clusters[v];
+            std::vector<ifc_config> probe(copies, rep);
+            for (ifc_config &c : probe) {
+                c.convection_scheme = IFC_CONV_UPWIND;  // the variants differ in their sweeps only
+                c.tol_u = c.tol_v = c.tol_w = c.tol_p = 0.0;
+                c.tol_mass = 0.0;
+                c.num_outer_iter = 20;
+                c.convection_scheme = IFC_CONV_UPWIND;
+            }
+            std::vector<ifc_batch_result> r(copies);
+            const std::vector<Plan> plan(copies, Plan{v, kVariantSweeps[v]});
+            ok = ok && batch_run<T>(probe.data(), copies, plan, r.data(), nullptr, &ms[q]) == IFC_OK;
+        }
+        if (!ok || !(ms[0] > 0.0)) continue;
+        t.done = true;
+        t.lone[v] = ms[0];
+        t.full[v] = std::max(ms[0], ms[1]);
+        const double per_case = t.full[v] / t.clusters[v];
+        if (best == 0.0 || per_case < best) {
+            best = per_case;
+            t.check = kVariantSweeps[v];
+        }
         if (getenv("IFC_VERBOSE"))
-            fprintf(stderr, "ifc_batch autotune: class %d (%dx%d) variant %d: %.3f ms\n", cls, rep.nx, rep.ny, v, ms);
+            fprintf(stderr, "ifc_batch autotune: class %d (%dx%d) variant %d: %.3f ms alone, %.3f ms on %d clusters\n", cls,
+                    rep.nx, rep.ny, v, ms[0], ms[1], t.clusters[v]);
     }
     return t;
 }
@@ -676,15 +781,24 @@ static Tuned autotune(int cls, const ifc_config &rep)
 template <typename T>
 static int batch_solve(const ifc_config *cfgs, int n, ifc_batch_result *res, void *const *fields_out, double *ms_out)
 {
-    const char *env = getenv("IFC_BATCH_VARIANT");
-    if (env && env[0] >= '0' && env[0] < '0' + kNumVariants)
-        return batch_run<T>(cfgs, n, std::vector<int>(n, env[0] - '0'), res, fields_out, ms_out);
+    std::vector<Plan> plan(n);
+    // only the whole-row kernel applies the deferred correction
+    auto whole_rows = [&](int c) { return cfgs[c].convection_scheme != IFC_CONV_UPWIND; };
+    const char *env = getenv("IFC_BATCH_VARIANT"), *env_check = getenv("IFC_BATCH_CHECK");
+    const int check = env_check ? std::max(0, std::atoi(env_check)) : 0;
+    if (env && env[0] >= '0' && env[0] < '0' + kNumVariants) {
+        const int v = env[0] - '0';
+        for (int c = 0; c < n; ++c)
+            if (!whole_rows(c)) plan[c] = {v, check > 0 ? check : kVariantSweeps[v]};
+        return batch_run<T>(cfgs, n, plan, res, fields_out, ms_out);
+    }
     const int prec = sizeof(T) == 8 ? 1 : 0;
-    std::vector<int> wanted(n, 0);
+    std::vector<ClassWork> work;
+    std::vector<int> at(kNumClasses, -1);
     for (int cls = 0; cls < kNumClasses; ++cls) {
         std::vector<int> members;
         for (int c = 0; c < n; ++c)
-            if (size_class(cfgs[c].nx, cfgs[c].ny) == cls) members.push_back(c);
+            if (!whole_rows(c) && size_class(cfgs[c].nx, cfgs[c].ny) == cls) members.push_back(c);
         if (members.empty()) continue;
         std::sort(members.begin(), members.end(), [&](int x, int y) {
             return (long long)cfgs[x].nx * cfgs[x].ny < (long long)cfgs[y].nx * cfgs[y].ny;
@@ -697,22 +811,32 @@ static int batch_solve(const ifc_config *cfgs, int n, ifc_batch_result *res, voi
         if (!t.done) {
             t = autotune<T>(cls, cfgs[members[members.size() / 2]]);
             std::lock_guard<std::mutex> lk(g_tune_mu);
-            g_tuned[prec][cls] = t;
+            // two threads may have measured: the first one's choice stays
+            if (g_tuned[prec][cls].done) t = g_tuned[prec][cls];
+            else if (t.done) g_tuned[prec][cls] = t;
         }
-        std::vector<double> cells;
-        for (int c : members) cells.push_back((double)cfgs[c].nx * cfgs[c].ny);
-        const int v = choose_variant(t, cells);
-        for (int c : members) wanted[c] = v;
+        if (!t.done) continue;  // nothing could be measured: whole rows, tried again by the next call
+        ClassWork cw;
+        cw.t = t;
+        for (int c : members) cw.grids.push_back({cfgs[c].nx, cfgs[c].ny});
+        at[cls] = (int)work.size();
+        work.push_back(cw);
     }
-    return batch_run<T>(cfgs, n, wanted, res, fields_out, ms_out);
+    if (!work.empty()) {
+        const std::vector<int> choice = choose_variants<T>(work);
+        for (int c = 0; c < n; ++c) {
+            const int k = whole_rows(c) ? -1 : at[size_class(cfgs[c].nx, cfgs[c].ny)];
+            if (k >= 0) plan[c] = {choice[k], check > 0 ? check : work[k].t.check};
+        }
+    }
+    return batch_run<T>(cfgs, n, plan, res, fields_out, ms_out);
 }
 
-// Solves the cases, case c with variant wanted[c]; the cases of a variant are one
+// Solves the cases, case c as plan[c] says; the cases of a variant are one
 // persistent launch relaunched by a CUDA graph WHILE node.
 template <typename T>
-static int batch_run(const ifc_config *cfgs, int n, const std::vector<int> &wanted, ifc_batch_result *res,
-                     void *const *fields_out,
-                     double *ms_out)
+static int batch_run(const ifc_config *cfgs, int n, const std::vector<Plan> &plan, ifc_batch_result *res,
+                     void *const *fields_out, double *ms_out)
 {
     int rc = IFC_OK;
     std::vector<BCase<T>> hc(n);
@@ -736,8 +860,8 @@ static int batch_run(const ifc_config *cfgs, int n, const std::vector<int> &want
         for (int f = 0; f < 4; ++f) closed = closed && cfgs[c].vel_bc_type[f] != IFC_OUTLET;
         b.pin = cfgs[c].pin_pressure == 1 || (cfgs[c].pin_pressure < 0 && closed);
         b.max_outer = cfgs[c].num_outer_iter;
-        // only the whole-row kernel applies the deferred correction
-        variant[c] = cfgs[c].convection_scheme != IFC_CONV_UPWIND ? 0 : wanted[c];
+        b.check = plan[c].check;
+        variant[c] = plan[c].variant;
     }
     // One queue per variant, largest grids first (longest-processing-time
     // heuristic); the queue with the most work runs first.
@@ -789,8 +913,9 @@ static int batch_run(const ifc_config *cfgs, int n, const std::vector<int> &want
         const size_t cell_bytes = padded(nc * sizeof(T));
         const size_t total = n_cell * cell_bytes + padded(nuf * sizeof(T)) + padded(nvf * sizeof(T)) +
                              padded(n * sizeof(BCase<T>)) + padded(n * sizeof(BState)) + padded(sizeof(BQueue));
+        BCK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
         BCK(cudaMalloc(&slab, total));
-        BCK(cudaMemset(slab, 0, total));
+        BCK(cudaMemsetAsync(slab, 0, total, st));
         unsigned char *at = static_cast<unsigned char *>(slab);
         auto take = [&](size_t bytes) {
             void *q = at;
@@ -803,8 +928,7 @@ static int batch_run(const ifc_config *cfgs, int n, const std::vector<int> &want
         dcases = static_cast<BCase<T> *>(take(n * sizeof(BCase<T>)));
         dstates = static_cast<BState *>(take(n * sizeof(BState)));
         dq = static_cast<BQueue *>(take(sizeof(BQueue)));
-        BCK(cudaMemcpy(dcases, queued.data(), n * sizeof(BCase<T>), cudaMemcpyHostToDevice));
-        BCK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+        BCK(cudaMemcpyAsync(dcases, queued.data(), n * sizeof(BCase<T>), cudaMemcpyHostToDevice, st));
         BCK(cudaEventCreate(&e0));
         BCK(cudaEventCreate(&e1));
         const int chunk = 250;
@@ -818,7 +942,7 @@ static int batch_run(const ifc_config *cfgs, int n, const std::vector<int> &want
             if (nclusters > qsize[gq]) nclusters = qsize[gq];
             if (getenv("IFC_VERBOSE"))
                 fprintf(stderr, "ifc_batch_solve: queue of %d cases, variant %d, %d clusters of %d CTAs\n", qsize[gq],
-                        v, nclusters, kCL);
+                        v, nclusters, variant_launch<T>(v).cl);
             cudaGraph_t graph = nullptr;
             cudaGraphExec_t exec = nullptr;
             cudaGraphConditionalHandle cond;
@@ -867,7 +991,7 @@ static int batch_run(const ifc_config *cfgs, int n, const std::vector<int> &want
             const VariantLaunch vl = variant_launch<T>(variant[c]);
             r.tile_x = vl.tx;
             r.tile_y = vl.ty;
-            r.sweeps_per_pass = kVariantSweeps[variant[c]];
+            r.sweeps_per_pass = plan[c].check;
             if (fields_out && fields_out[c]) {
                 const size_t cells = (size_t)cfgs[c].nx * cfgs[c].ny;
                 T *out = (T *)fields_out[c];

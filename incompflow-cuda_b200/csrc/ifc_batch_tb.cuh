@@ -13,12 +13,12 @@
 // passes and phases; every norm is reduced per CTA in a fixed order and across
 // the cluster through distributed shared memory in rank order, so each CTA
 // takes the same early-exit and convergence decisions.  The region shape, the
-// cluster size and the sweeps per pass distinguish the variants; the batch
-// autotuner picks one per size class.  Against whole-row sweeps (a cluster
-// barrier per half sweep, every coefficient rebuilt from L1/L2 in every half
-// sweep) a batch of 48 cavities of 32..256 squared takes 67 ms instead of 102
-// for 60 iterations each; a batch of hundreds keeps all of the whole-row form's
-// 71 clusters busy and stays with it.
+// cluster size and the sweeps per pass distinguish the variants; a batch picks
+// them by its cases.  Against whole-row sweeps (a cluster barrier per half sweep,
+// every coefficient rebuilt from L1/L2 in every half sweep) a batch of 48
+// cavities of 32..256 squared takes 51 ms instead of 92 for 60 iterations each; a
+// batch of hundreds of them keeps all of the whole-row form's 71 clusters busy
+// and stays with it (256 cavities, 40 iterations: 134 ms, 184 in variant 2).
 
 template <typename T>
 struct TBPools {
@@ -49,21 +49,19 @@ __device__ __forceinline__ void tb_cluster_total(cg::cluster_group &cl, double *
     __syncthreads();
 }
 
-// Inner early-exit rule (src/Solver.cu:955-962) after a pass of ns sweeps with
-// per-sweep sums sq[0..ns).
-__device__ __forceinline__ void tb_pass_done(CaseLoop &L, int e, const double *sq, int ns, int N, double tol)
+// After a pass of ns sweeps of equation e from sweep `first`, with per-sweep
+// sums sq[0..ns): the early-exit rule (not a second time when the pass was run
+// `again`).
+__device__ __forceinline__ void tb_pass_done(CaseLoop &L, int e, const double *sq, int first, int ns, int n, int check,
+                                             int N, double tol, bool again)
 {
-    double mx = L.inner_max[e];
-    bool stop_now = false;
-    for (int s = 0; s < ns && !stop_now; ++s) {
-        const double rms = sqrt(sq[s] / (double)N);
-        if (rms > mx) mx = rms;
-        if (rms / (mx + 1e-20) < tol) stop_now = true;
-    }
-    L.inner_max[e] = mx;
-    L.sweeps[e] += ns;
-    if (stop_now) L.stop[e] = 1;
+    if (ns == 0) return;
+    for (int s = 0; s < ns && !L.hit[e] && !again; ++s) inner_rule(L, e, sq[s], first + s, n, check, N, tol);
+    L.sweeps[e] = first + ns;
 }
+
+// Sweeps of a pass that starts at sweep `first` of an inner solve of `limit`.
+__device__ __forceinline__ int tb_sweeps(int limit, int first, int ks) { return max(0, min(limit - first, ks)); }
 
 // Rhie-Chow velocity of interior face k of n along its axis (stride st; c: the
 // cell above the face), with the reciprocals of the diagonals.
@@ -175,7 +173,8 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(32 * NW_, 1)
         for (int it = 0; it < chunk && !S.done; ++it) {
             if (tid == 0)
                 for (int e = 0; e < 4; ++e) {
-                    L.stop[e] = 0;
+                    L.limit[e] = C.n_iter[e];
+                    L.hit[e] = 0;
                     L.inner_max[e] = -1e20;
                     L.sweeps[e] = 0;
                 }
@@ -183,13 +182,13 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(32 * NW_, 1)
             int mcur = 0, pcur = 0;
 
             // ---------------- momentum passes ----------------
-            const int nu = C.n_iter[0], nv = C.n_iter[1];
-            const int npass_m = (max(nu, nv) + KS - 1) / KS;
-            for (int pass = 0; pass < (npass_m > 0 ? npass_m : 1); ++pass) {
-                const int ns0 = clamp_sweeps(nu, pass, KS), ns1 = clamp_sweeps(nv, pass, KS);
-                const bool au = ns0 > 0 && !L.stop[EQ_U];
-                const bool av = ns1 > 0 && !L.stop[EQ_V];
-                if (!au && !av && pass > 0) continue;  // the same in every CTA
+            // (When the early-exit rule ends an inner solve before its pass does -- the
+            // case is checked more often than KS sweeps -- the pass is run
+            // again, from the same values, with fewer sweeps.)
+            bool again = false;
+            for (int first = 0;;) {
+                const int ns0 = tb_sweeps(L.limit[EQ_U], first, KS), ns1 = tb_sweeps(L.limit[EQ_V], first, KS);
+                if (ns0 == 0 && ns1 == 0 && first > 0) break;  // the same in every CTA
 #pragma unroll 1
                 for (int t = (int)rank; t < ntiles; t += CL) {
                     const LanePlace<RT> pl(tile_box(tg, t, nx, ny), ny);
@@ -198,12 +197,12 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(32 * NW_, 1)
                     load_cells<RT, T>(cu, bu[mcur], pl, nx, ny, false, kOutside<T>);
                     load_cells<RT, T>(cv, bv[mcur], pl, nx, ny, false, kOutside<T>);
                     const bool force = mom_links<RT, T>(P, f, pl, a);
-                    if (pass == 0) store_diagonal<RT, T>(a, ac, rac, pl, nx);
+                    if (first == 0) store_diagonal<RT, T>(a, ac, rac, pl, nx);
                     publish<RT, T>(cu, 0);
                     publish<RT, T>(cv, 1);
                     __syncthreads();
-                    sweeps2<RT, T>(cu, cv, a, pl, g.relax[EQ_U], g.relax[EQ_V], force, au ? ns0 : 0, av ? ns1 : 0, KS,
-                                   true, t != (int)rank, sred);
+                    sweeps2<RT, T>(cu, cv, a, pl, g.relax[EQ_U], g.relax[EQ_V], force, ns0, ns1, KS, true,
+                                   t != (int)rank, sred);
                     store_own<RT, T>(cu, bu[mcur ^ 1], pl, nx);
                     store_own<RT, T>(cv, bv[mcur ^ 1], pl, nx);
                 }
@@ -212,11 +211,14 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(32 * NW_, 1)
                 tb_cluster_total<CL>(cl, part[rs], 2 * KS, tot);
                 rs ^= 1;
                 if (tid == 0) {
-                    if (au) tb_pass_done(L, EQ_U, tot, ns0, N, g.tol[EQ_U]);
-                    if (av) tb_pass_done(L, EQ_V, tot + KS, ns1, N, g.tol[EQ_V]);
+                    tb_pass_done(L, EQ_U, tot, first, ns0, C.n_iter[0], C.check, N, g.tol[EQ_U], again);
+                    tb_pass_done(L, EQ_V, tot + KS, first, ns1, C.n_iter[1], C.check, N, g.tol[EQ_V], again);
                 }
                 __syncthreads();
+                again = (ns0 > 0 && first + ns0 > L.limit[EQ_U]) || (ns1 > 0 && first + ns1 > L.limit[EQ_V]);
+                if (again) continue;
                 mcur ^= 1;
+                first += KS;
             }
             const T *const cu = bu[mcur], *const cv = bv[mcur];
 
@@ -249,17 +251,16 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(32 * NW_, 1)
             }
 
             // ---------------- p' passes from p' = 0 ----------------
-            const int np = C.n_iter[3];
-            const int npass_p = (np + KS - 1) / KS;
-            for (int pass = 0; pass < npass_p; ++pass) {
-                const int ns = clamp_sweeps(np, pass, KS);
-                if (ns <= 0 || L.stop[EQ_P]) continue;  // the same in every CTA
+            again = false;
+            for (int first = 0;;) {
+                const int ns = tb_sweeps(L.limit[EQ_P], first, KS);
+                if (ns == 0) break;  // the same in every CTA
 #pragma unroll 1
                 for (int t = (int)rank; t < ntiles; t += CL) {
                     const LanePlace<RT> pl(tile_box(tg, t, nx, ny), ny);
                     Links<RT, T> a;
                     Cells<T, R> x;
-                    if (pass == 0) zero_cells<RT, T>(x, pl, nx, ny);
+                    if (first == 0) zero_cells<RT, T>(x, pl, nx, ny);
                     else load_cells<RT, T>(x, bp[pcur], pl, nx, ny, false, kOutside<T>);
                     const bool force = pc_links<RT, T>(P, f, pl, a);
                     publish<RT, T>(x, 0);
@@ -271,12 +272,15 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(32 * NW_, 1)
                 cl.sync();
                 tb_cluster_total<CL>(cl, part[rs], KS, tot);
                 rs ^= 1;
-                if (tid == 0) tb_pass_done(L, EQ_P, tot, ns, N, g.tol[EQ_P]);
+                if (tid == 0) tb_pass_done(L, EQ_P, tot, first, ns, C.n_iter[3], C.check, N, g.tol[EQ_P], again);
                 __syncthreads();
+                again = first + ns > L.limit[EQ_P];
+                if (again) continue;
                 pcur ^= 1;
+                first += KS;
             }
             T *const pcc = bp[pcur];
-            if (npass_p == 0) {
+            if (C.n_iter[3] <= 0) {
                 for (int j = gw; j < ny; j += TW)
                     for (int i = lane; i < nx; i += 32) pcc[i + nx * j] = (T)0;
                 cl.sync();

@@ -91,3 +91,59 @@ def test_batch_rejects_3d_and_mixed_precision():
         keep.append(kp)
     res = (ifc.IfcBatchResult * 2)()
     assert ifc.load().ifc_batch_solve(arr, 2, res, None, None) == ifc.UNSUPPORTED
+
+
+def loose(cfg, **kw):
+    """Open domain (no p' mean, whose FP64 sum depends on the order of its terms)
+    and inner tolerances that end the sweeps early, at changing places."""
+    return dict(cfg, numOuterIter=3, nIter_u=13, nIter_v=11, nIter_p=23, tol_u=0.6, tol_v=0.6, tol_p=0.9,
+                criterion=O.CRIT_PER_FIELD, tol_mass=0.0, **kw)
+
+
+@pytest.mark.parametrize("prec", ["f", "d"])
+@pytest.mark.parametrize("check", [1, 2, 3, 4, 5, 7])
+def test_exit_interval_of_every_variant(gpu_ok, monkeypatch, prec, check):
+    """The inner early exit after every `check` sweeps, deeper and shallower than
+    the variants' passes: the oracle's sweep counts, and the same values from
+    every variant.  Tolerance: exact."""
+    monkeypatch.setenv("IFC_BATCH_CHECK", str(check))
+    cases = [loose(c, precision=prec) for c in (ifc.channel2d(64, 32), ifc.channel2d(97, 40), ifc.channel2d(30, 70))]
+    out = []
+    for variant in "012":
+        monkeypatch.setenv("IFC_BATCH_VARIANT", variant)
+        res, fields, _ = ifc.batch_solve(cases)
+        out.append((res, fields))
+    ended = 0
+    for k, c in enumerate(cases):
+        o = O.Oracle(to_oracle_cfg(dict(c, sweep_mode=O.GS_REDBLACK, check_every=check)), prec)
+        o.init_face_vel()
+        o.bc_face_vel()
+        done = 0
+        while done < out[0][0][k]["outer_iterations"]:
+            want = o.outer_iteration()["sweeps"]
+            o.bc_face_vel()
+            done += 1
+        ended += sum(want) < 13 + 11 + 23
+        for res, fields in out:
+            assert res[k]["sweeps_per_pass"] == check
+            assert res[k]["outer_iterations"] == done and list(res[k]["sweeps"]) == list(want), (k, res[k], want)
+            for f in ("u", "v", "p"):
+                assert np.array_equal(fields[k][f].ravel(), o.field(f)), (k, f)
+    assert ended  # some inner solves did end early
+
+
+@pytest.mark.parametrize("prec", ["f", "d"])
+def test_a_case_does_not_depend_on_its_batch(gpu_ok, monkeypatch, prec):
+    """The same cases in a small batch and among many others, which run them in
+    other variants: the same values and counts.  Tolerance: exact."""
+    monkeypatch.delenv("IFC_BATCH_VARIANT", raising=False)
+    cases = [loose(c, precision=prec) for c in (ifc.channel2d(64, 40), ifc.channel2d(140, 130), ifc.channel2d(230, 131))]
+    others = [loose(ifc.channel2d(150 + 3 * k, 140), precision=prec) for k in range(28)] * 5
+    r1, f1, _ = ifc.batch_solve(cases)
+    r2, f2, _ = ifc.batch_solve(others + cases)
+    for a, b, fa, fb in zip(r1, r2[len(others):], f1, f2[len(others):]):
+        assert (a["outer_iterations"], list(a["sweeps"]), a["sweeps_per_pass"]) == \
+               (b["outer_iterations"], list(b["sweeps"]), b["sweeps_per_pass"])
+        for f in ("u", "v", "p"):
+            assert np.array_equal(fa[f], fb[f]), f
+    assert any(a["tile_y"] != b["tile_y"] for a, b in zip(r1, r2[len(others):]))  # other variants did run them

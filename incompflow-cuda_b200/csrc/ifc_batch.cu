@@ -969,6 +969,16 @@ static int batch_run(const ifc_config *cfgs, int n, const std::vector<Plan> &pla
         BCK(cudaEventRecord(e1, st));
         BCK(cudaStreamSynchronize(st));
         BCK(cudaGetLastError());
+#ifdef IFC_BOUNDS_CHECK
+        int out_of_range = 0;
+        BCK(cudaMemcpyFromSymbol(&out_of_range, g_ifc_bounds_err, sizeof(int)));
+        if (out_of_range) {
+            const int zero = 0;
+            BCK(cudaMemcpyToSymbol(g_ifc_bounds_err, &zero, sizeof(int)));
+            rc = IFC_BAD_ARGUMENT;
+            goto done;
+        }
+#endif
         float ms = 0.f;
         BCK(cudaEventElapsedTime(&ms, e0, e1));
         if (ms_out) *ms_out = ms;

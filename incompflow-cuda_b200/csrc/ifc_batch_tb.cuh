@@ -194,17 +194,17 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(32 * NW_, 1)
                     const LanePlace<RT> pl(tile_box(tg, t, nx, ny), ny);
                     Links<RT, T> a;
                     Cells<T, R> cu, cv;
-                    load_cells<RT, T>(cu, bu[mcur], pl, nx, ny, false, kOutside<T>);
-                    load_cells<RT, T>(cv, bv[mcur], pl, nx, ny, false, kOutside<T>);
+                    load_cells<RT, T>(cu, field_view(bu[mcur], N), pl, nx, ny, false, kOutside<T>);
+                    load_cells<RT, T>(cv, field_view(bv[mcur], N), pl, nx, ny, false, kOutside<T>);
                     const bool force = mom_links<RT, T>(P, f, pl, a);
-                    if (first == 0) store_diagonal<RT, T>(a, ac, rac, pl, nx);
+                    if (first == 0) store_diagonal<RT, T>(a, field_view(ac, N), field_view(rac, N), pl, nx);
                     publish<RT, T>(cu, 0);
                     publish<RT, T>(cv, 1);
                     __syncthreads();
                     sweeps2<RT, T>(cu, cv, a, pl, g.relax[EQ_U], g.relax[EQ_V], force, ns0, ns1, KS, true,
                                    t != (int)rank, sred);
-                    store_own<RT, T>(cu, bu[mcur ^ 1], pl, nx);
-                    store_own<RT, T>(cv, bv[mcur ^ 1], pl, nx);
+                    store_own<RT, T>(cu, field_view(bu[mcur ^ 1], N), pl, nx);
+                    store_own<RT, T>(cv, field_view(bv[mcur ^ 1], N), pl, nx);
                 }
                 tb_part<NT>(sred, 2 * KS, ntiles > (int)rank, part[rs]);
                 cl.sync();
@@ -261,12 +261,12 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(32 * NW_, 1)
                     Links<RT, T> a;
                     Cells<T, R> x;
                     if (first == 0) zero_cells<RT, T>(x, pl, nx, ny);
-                    else load_cells<RT, T>(x, bp[pcur], pl, nx, ny, false, kOutside<T>);
+                    else load_cells<RT, T>(x, field_view(bp[pcur], N), pl, nx, ny, false, kOutside<T>);
                     const bool force = pc_links<RT, T>(P, f, pl, a);
                     publish<RT, T>(x, 0);
                     __syncthreads();
                     sweeps1<RT, T>(x, a, pl, g.relax[EQ_P], force, ns, KS, true, t != (int)rank, sred);
-                    store_own<RT, T>(x, bp[pcur ^ 1], pl, nx);
+                    store_own<RT, T>(x, field_view(bp[pcur ^ 1], N), pl, nx);
                 }
                 tb_part<NT>(sred, KS, ntiles > (int)rank, part[rs]);
                 cl.sync();

@@ -71,9 +71,20 @@ struct Checked {
 };
 template <typename T>
 using FieldArr = Checked<T>;
+template <typename T>
+__device__ __forceinline__ FieldArr<T> field_view(T *p, long long n)
+{
+    return {p, n};
+}
 #else
 template <typename T>
 using FieldArr = T *;
+// n values at p as a field array.
+template <typename T>
+__device__ __forceinline__ FieldArr<T> field_view(T *p, long long)
+{
+    return p;
+}
 #endif
 
 template <typename T>

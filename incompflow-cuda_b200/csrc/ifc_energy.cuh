@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(32 * NW_, 1)
 
     bool failed = false;
     unsigned int epoch = 0;
-    auto buf = [&](int q) { return q ? x1 : x0; };
+    auto buf = [&](int q) { return field_view(q ? x1 : x0, N); };
     int cur = 0, set = 0;
     Pending pending;
     pending.kind = kPendNone;
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(32 * NW_, 1)
     }
     __syncthreads();
     // the last stored pass read x0, and every CTA has passed its barrier
-    if (!failed && cur == 1) store_other<RT, T>(x0, x1, pl, nx);
+    if (!failed && cur == 1) store_other<RT, T>(buf(0), buf(1), pl, nx);
     if (blockIdx.x == 0 && tid == 0 && !failed) {
         const double top = L.inner_max_sq[eq] >= 0.0 ? sqrt(L.inner_max_sq[eq] / (double)N) : -1e20;
         ctl->inner_max[eq] = top > floor ? top : floor;

@@ -444,9 +444,9 @@ __global__ void __launch_bounds__(32 * NW_, 1) k_simple2d(const __grid_constant_
     // A pass stages halos from one buffer and writes its tile to the other, so
     // no tile reads a neighbour tile's values of the same pass; `mcur`/`pcur`
     // (the same in every CTA) say which buffer holds the current u, v / p'.
-    auto bu = [&](int q) -> T * { return q ? (T *)f.tmp : (T *)f.u; };
-    auto bv = [&](int q) -> T * { return q ? (T *)f.tmp + N : (T *)f.v; };
-    auto bp = [&](int q) -> T * { return q ? (T *)f.tmp + 2 * (size_t)N : (T *)f.pc; };
+    auto bu = [&](int q) { return field_view(q ? (T *)f.tmp : (T *)f.u, N); };
+    auto bv = [&](int q) { return field_view(q ? (T *)f.tmp + N : (T *)f.v, N); };
+    auto bp = [&](int q) { return field_view(q ? (T *)f.tmp + 2 * (size_t)N : (T *)f.pc, N); };
 
     const LanePlace<RT> place(tile_box(pa.tiles, blockIdx.x, nx, ny), ny);  // in the CTA's first tile
     Pending pending;
@@ -690,7 +690,7 @@ __global__ void __launch_bounds__(32 * NW_, 1) k_simple2d(const __grid_constant_
         }
         if (failed) break;
 
-        T *const pcc = bp(pcur);  // the current p'
+        const FieldArr<T> pcc = bp(pcur);  // the current p'
         if (npass_p == 0) {       // no p' sweeps: p' = 0 (src/Solver.cu:193)
             // no p' pass takes a decision left over from the momentum passes
             if (pending.kind) resolve_now();

@@ -534,8 +534,8 @@ struct LanePlace {
 
 // x = field[cell] of the lane's cells (`outside` beyond the domain); with
 // only_halo, the tile's own cells keep their values.
-template <typename RT, typename T>
-__device__ __forceinline__ void load_cells(Cells<T, RT::R> &x, const T *field, const LanePlace<RT> &pl, int nx, int ny,
+template <typename RT, typename T, typename A>
+__device__ __forceinline__ void load_cells(Cells<T, RT::R> &x, const A &field, const LanePlace<RT> &pl, int nx, int ny,
                                            bool only_halo, T outside)
 {
 #pragma unroll
@@ -550,8 +550,8 @@ __device__ __forceinline__ void load_cells(Cells<T, RT::R> &x, const T *field, c
     }
 }
 
-template <typename RT, typename T>
-__device__ __forceinline__ void store_own(const Cells<T, RT::R> &x, T *field, const LanePlace<RT> &pl, int nx)
+template <typename RT, typename T, typename A>
+__device__ __forceinline__ void store_own(const Cells<T, RT::R> &x, const A &field, const LanePlace<RT> &pl, int nx)
 {
 #pragma unroll
     for (int r = 0; r < RT::R; ++r) {
@@ -563,8 +563,8 @@ __device__ __forceinline__ void store_own(const Cells<T, RT::R> &x, T *field, co
 }
 
 // to = from on the tile's own cells.
-template <typename RT, typename T>
-__device__ __forceinline__ void store_other(T *to, const T *from, const LanePlace<RT> &pl, int nx)
+template <typename RT, typename T, typename A>
+__device__ __forceinline__ void store_other(const A &to, const A &from, const LanePlace<RT> &pl, int nx)
 {
 #pragma unroll
     for (int r = 0; r < RT::R; ++r) {
@@ -726,8 +726,9 @@ __device__ __forceinline__ bool mom_links(const Params<T> &P, const Fields<T> &f
 
 // The momentum diagonal of the tile's own cells and its reciprocal to global
 // memory (the reciprocals serve Rhie-Chow, the p' links and the corrections).
-template <typename RT, typename T>
-__device__ __forceinline__ void store_diagonal(const Links<RT, T> &a, T *ac, T *rac, const LanePlace<RT> &pl, int nx)
+template <typename RT, typename T, typename A>
+__device__ __forceinline__ void store_diagonal(const Links<RT, T> &a, const A &ac, const A &rac, const LanePlace<RT> &pl,
+                                               int nx)
 {
     Cells<T, RT::R> c;
 #pragma unroll

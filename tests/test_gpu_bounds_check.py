@@ -29,3 +29,15 @@ def test_parity_tests_pass_under_the_bounds_checked_build(gpu_ok):
                        env=env, cwd=ROOT, capture_output=True, text=True, timeout=1200)
     assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-2000:]
     assert " passed" in r.stdout
+
+
+def test_region_and_batch_tests_pass_under_the_bounds_checked_build(gpu_ok):
+    """The same for the regions held in registers, whose loads and stores go
+    through the checked arrays, and for the batched solves, which report an
+    index out of range in the same way."""
+    env = dict(os.environ, IFC_LIB=LIB_BC)
+    r = subprocess.run([sys.executable, "-m", "pytest", "-q", "-x", "-m", "gpu", "-p", "no:cacheprovider",
+                        "tests/test_gpu_tile2d.py", "tests/test_gpu_batch.py", "tests/test_gpu_quotient_range.py"],
+                       env=env, cwd=ROOT, capture_output=True, text=True, timeout=1200)
+    assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-2000:]
+    assert " passed" in r.stdout

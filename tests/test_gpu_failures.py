@@ -83,3 +83,22 @@ def test_3d_cooperative_timeout_is_reported_at_sync_and_handle_stays_usable(gpu_
     st = s.iterate(3)
     assert st["status"] == ifc.OK and st["outer_iterations"] == 8
     assert np.isfinite(s.get("u")).all()
+
+
+def test_3d_pressure_rows_timeout_is_reported_at_sync_and_handle_stays_usable(gpu_ok, monkeypatch):
+    """The same with rows long enough for k_psolve3d, whose even half sweeps
+    arrive at the grid barrier and wait for it in two steps."""
+    s = ifc.Solver(dict(ifc.cavity3d(16), nx=77, ny=31, nz=30))
+    s.iterate(2)
+    s.stage("mom_solve")
+    s.stage("rhie_chow")
+    monkeypatch.setenv("IFC_TEST_STALL_BARRIER", "1")
+    s.stage("pcorr_solve", wait=False)
+    with pytest.raises(ifc.IfcError) as e:
+        s.sync()
+    assert e.value.status == ifc.TIMEOUT
+    monkeypatch.delenv("IFC_TEST_STALL_BARRIER")
+    s.stage("pcorr_solve")
+    st = s.iterate(3)
+    assert st["status"] == ifc.OK and st["outer_iterations"] == 5
+    assert np.isfinite(s.get("u")).all()

@@ -9,7 +9,7 @@ import pytest
 
 import ifc
 import oracle as O
-from helpers import assert_bitwise, load_both, seeded_state, to_oracle_cfg
+from helpers import assert_bitwise, load_both, rel_l2, seeded_state, to_oracle_cfg
 
 pytestmark = pytest.mark.gpu
 
@@ -196,3 +196,60 @@ def test_small_and_narrow_regions(gpu_ok, nx, ny, spp, prec):
     """Regions of 20 and 28 rows: filled exactly, one row more, and the tall
     narrow grid that takes them at the default depth."""
     check(dict(ifc.channel2d(nx, ny), precision=prec, sweeps_per_pass=spp), 2)
+
+
+@pytest.mark.parametrize("prec,bound", [("f", 1e-6), ("d", 1e-11)])
+def test_several_tiles_per_cta_closed(gpu_ok, monkeypatch, prec, bound):
+    """Several tiles per CTA with the p' mean removal of a closed domain (150
+    columns are at least three tiles, on two CTAs).  Relative L2 against the
+    oracle: the values differ by the order of the mean's FP64 sum only, at most
+    15150 terms times the rounding unit (FP64), less than one FP32 rounding."""
+    monkeypatch.setenv("IFC_PERSIST_MAX_CTAS", "2")
+    cfg = dict(ifc.cavity2d(150, ny=101), precision=prec)
+    o = O.Oracle(to_oracle_cfg(cfg), prec)
+    s = ifc.Solver(cfg)
+    load_both(o, s, seeded_state(cfg, 3, s.dtype))
+    for it in range(3):
+        assert s.iterate(1)["kernel_launches"] == 3
+        o.outer_iteration()
+        o.bc_face_vel()
+        for k in ("u", "v", "p", "uf", "vf"):
+            assert rel_l2(s.get(k), o.field(k)) < bound, (it, k)
+
+
+def test_several_tiles_per_cta_converged(gpu_ok, monkeypatch):
+    """A cavity to convergence with several tiles per CTA (130 columns are at
+    least three tiles) against one tile per CTA: the per-sweep FP64 sums are
+    grouped by CTA, so only their rounding can differ."""
+    cfg = ifc.cavity2d(130, ny=40)
+    one = ifc.Solver(cfg)
+    a = one.solve()
+    monkeypatch.setenv("IFC_PERSIST_MAX_CTAS", "2")
+    several = ifc.Solver(cfg)
+    b = several.solve()
+    assert a["converged"] and b["converged"] and abs(a["outer_iterations"] - b["outer_iterations"]) <= 2
+    for k in ("u", "v"):
+        assert rel_l2(several.get(k), one.get(k)) < 1e-6, k
+
+
+@pytest.mark.parametrize("nx,ny,nz,prec", [(80, 128, 128, "f"), (77, 100, 103, "d")])
+def test_3d_pressure_blocks(gpu_ok, monkeypatch, nx, ny, nz, prec):
+    """The 3D p' solve on blocks with inner rows (ny*nz rows on at most 148 blocks:
+    70 and more rows each, 10x12 and 8x9), so rows whose four neighbours are in
+    shared memory, and the sweep of inner rows between the two halves of the
+    grid barrier; against the per-half-sweep kernels.  Tolerance: exact."""
+    cfg = dict(ifc.cavity3d(16), nx=nx, ny=ny, nz=nz, precision=prec, nIter_p=9)
+    state = seeded_state(cfg, 4, np.float32 if prec == "f" else np.float64)
+    for tol in (0.0, 0.3):
+        out = []
+        for off in ("0", "1"):
+            monkeypatch.setenv("IFC_PC3D_OFF", off)
+            s = ifc.Solver(dict(cfg, tol_p=tol, pin_pressure=0))
+            for k, v in state.items():
+                s.set(k, v)
+            r = s.iterate(1)
+            out.append((list(r["sweeps"]), [s.get(k) for k in ("pc", "p", "u", "v", "w", "uf")]))
+            s.close()
+        assert out[0][0] == out[1][0]
+        for k, a, b in zip(("pc", "p", "u", "v", "w", "uf"), out[0][1], out[1][1]):
+            assert_bitwise(a, b, f"tol {tol} {k}")

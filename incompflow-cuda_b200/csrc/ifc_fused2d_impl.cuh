@@ -158,37 +158,41 @@ void Engine<T>::enq_fused_rc()
 namespace ifc {
 
 // ---- the persistent single-launch 2D solve (ifc_persist2d.cuh) ----
-// Region shapes: rows per lane and warps (a region is 64 x R*NW cells).  The
-// shape with the least estimated time per pass is taken: rounds of tiles per
-// CTA times the shape's cost of a pass (relative time of a half sweep).  Small
-// grids leave SMs idle, so the smallest region with the shortest half sweep
-// wins as long as its tiles fit one round (64x64 cavity: 69 ms to convergence
-// with 24 rows, 77 with 32; FP64 500x36: 113 against 148 us per iteration);
-// the larger regions waste less on halos and win once they save a round
-// (1024x256: 112 us with 64 rows; 32 rows would take 4 rounds).  FP64 has half
-// the registers per cell: 64 rows do not fit, 36 rows (500x190 in one round)
-// do; its half sweeps take in proportion to their rows (64x64, us per outer
-// iteration with 24, 28, 32 and 36 rows: 67, 76, 85, 106), so a single tile gains
-// little from having no barriers (33x31: 79 us in one of 32 rows, 65 in three of
-// 24), 20 rows serve passes of up to four sweeps (33x31, 4 sweeps: 88 -> 70) and
-// 28 rows tall grids that 24 do not hold in one round (29x621: 83 -> 77; FP32 56
-// -> 54).
+// Region shapes: rows per lane and warps (a region is 64 x R*NW cells), and the
+// relative time of an outer iteration with one tile per CTA (`one`) or with n in
+// turn, whose links are rebuilt in every pass (base + n * each); the shape with
+// the least is taken.  In us of the 5-sweep channel, FP32 / FP64, one tile: 24
+// rows 50 / 68, 28 rows 54 / 76, 32 rows 57 / 84, 36 rows - / 101, 64 rows 105 /
+// -.  Two tiles: 24 rows 90 FP32, 28 rows 106 FP32, 32 rows 111 / 175, 36 rows -
+// / 211, 64 rows 228 FP32; eight of 28 rows 315 / 493, six of 32 268 / 437, four
+// of 36 - / 374.  So small grids, which leave SMs idle, take the smallest region
+// whose tiles fit one round, and the larger regions, which waste less on halos,
+// win once they save rounds (1024x256: 106 us in one round of 64 rows).  FP64
+// has half the registers per cell: 64 rows do not fit.  Its half sweeps take in
+// proportion to their rows, so a single tile gains little from having no
+// barriers (33x31: 79 us in one of 32 rows, 65 in three of 24), and 20 rows serve
+// passes of up to four sweeps (33x31, 4 sweeps: 88 -> 70).
 struct RegionShape {
     int R, NW;
-    double cost;
+    double one, base, each;
 };
 template <typename T>
 struct RegionShapes;
 template <>
 struct RegionShapes<float> {
     static constexpr int n = 4;
-    static constexpr RegionShape s[n] = {{2, 12, 0.85}, {2, 14, 0.92}, {2, 16, 1.0}, {4, 16, 1.6}};
-    static constexpr double alone = 0.3;  // what a pass gains without grid barriers
+    static constexpr RegionShape s[n] = {
+        {2, 12, 0.87, 0.46, 0.56}, {2, 14, 0.95, 0.60, 0.61}, {2, 16, 1.0, 0.58, 0.68}, {4, 16, 1.85, 0.30, 1.80}};
+    static constexpr double alone = 0.3;  // what a single tile gains without grid barriers
 };
 template <>
 struct RegionShapes<double> {
     static constexpr int n = 5;
-    static constexpr RegionShape s[n] = {{2, 10, 0.7}, {2, 12, 0.8}, {2, 14, 0.9}, {2, 16, 1.0}, {2, 18, 1.2}};
+    static constexpr RegionShape s[n] = {{2, 10, 0.70, 0.45, 0.42},
+                                         {2, 12, 0.80, 0.47, 0.50},
+                                         {2, 14, 0.90, 0.54, 0.67},
+                                         {2, 16, 1.0, 0.54, 0.77},
+                                         {2, 18, 1.2, 0.56, 0.98}};
     static constexpr double alone = 0.1;
 };
 
@@ -314,7 +318,7 @@ int Engine<T>::prepare_persist()
             const int passes = (n_m + pa.ks - 1) / pa.ks + (cfg.n_iter_p + pa.ks - 1) / pa.ks;
             // (a single tile runs without grid barriers)
             const double cost = (passes > 0 ? passes : 1) * (0.5 + 0.1 * pa.ks) *
-                                ((double)per * sh.cost - (tiles == 1 ? RegionShapes<T>::alone : 0.0));
+                                (per > 1 ? sh.base + (double)per * sh.each : tiles > 1 ? sh.one : sh.one - RegionShapes<T>::alone);
             if (persist && cost >= best) continue;
             best = cost;
             best_ks = pa.ks;
@@ -325,6 +329,28 @@ int Engine<T>::prepare_persist()
             pa.group = group;
         }
     pa.ks = best_ks;
+    if (!persist) return IFC_OK;
+    // SMs that have no tile: narrower tiles, of twelve columns and more, share out
+    // the phases between the sweeps (deferred correction, faces, corrections),
+    // whose time follows a CTA's own cells; the sweeps cost the same, a region
+    // each.  us per outer iteration, FP64 / FP32: 1169x18 QUICK 83 -> 73 / 62 -> 57,
+    // 64x64 68 -> 63 / 50 -> 48.  A single tile only where these phases outweigh
+    // its lack of barriers (64x22: FP64 QUICK 75 -> 73, FP64 upwind 64 -> 66, FP32
+    // 42 -> 50).
+    TileGrid &tg = pa.tiles;
+    const int tiles = tg.kx * tg.ky, inner = P.g.nx - 2 * tg.H;
+    int room = nsm;
+    if (cap_env > 0 && room > cap_env) room = cap_env;
+    if (persist_grid != tiles || inner <= 12 || (tiles == 1 && (sizeof(T) == 4 || cfg.convection_scheme == IFC_CONV_UPWIND)))
+        return IFC_OK;
+    const int most = room / tg.ky;
+    if (most <= tg.kx) return IFC_OK;
+    int w = (inner + most - 1) / most;
+    w += w & 1;
+    if (w < 12) w = 12;
+    tg.Ix = w;
+    tg.kx = (inner + w - 1) / w;
+    persist_grid = tg.kx * tg.ky;
     return IFC_OK;
 }
 
@@ -391,7 +417,7 @@ bool Engine<T>::coef_coop()
         if (!split_axis(P.g.nx, 64, tg.H, &tg.kx, &tg.Ix) || !split_axis(P.g.ny, sh.R * sh.NW, tg.H, &tg.ky, &tg.Iy))
             continue;
         const long long tiles = (long long)tg.kx * tg.ky;
-        const double cost = sh.cost - (tiles == 1 ? RegionShapes<T>::alone : 0.0);
+        const double cost = sh.one - (tiles == 1 ? RegionShapes<T>::alone : 0.0);
         int capacity = 0;
         if (coef_dispatch<T>(*this, s, nullptr, &capacity) != cudaSuccess) {
             cudaGetLastError();

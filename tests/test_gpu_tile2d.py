@@ -253,3 +253,14 @@ def test_3d_pressure_blocks(gpu_ok, monkeypatch, nx, ny, nz, prec):
         assert out[0][0] == out[1][0]
         for k, a, b in zip(("pc", "p", "u", "v", "w", "uf"), out[0][1], out[1][1]):
             assert_bitwise(a, b, f"tol {tol} {k}")
+
+
+@pytest.mark.parametrize("prec,conv", [("f", "upwind"), ("d", "upwind"), ("d", "quick")])
+@pytest.mark.parametrize("nx,ny,cap", [(32, 40, 0), (33, 40, 0), (46, 25, 0), (307, 19, 0), (64, 22, 0), (64, 64, 7), (111, 30, 5)])
+def test_narrow_tiles(gpu_ok, monkeypatch, nx, ny, cap, prec, conv):
+    """Tiles made narrower to use more CTAs: columns that just do not and just do
+    split into tiles of twelve, an odd last tile, one row of tiles, a cap on
+    the CTAs that leaves room for some of them."""
+    if cap:
+        monkeypatch.setenv("IFC_PERSIST_MAX_CTAS", str(cap))
+    check(dict(ifc.channel2d(nx, ny), precision=prec, convection_scheme=conv), 2)

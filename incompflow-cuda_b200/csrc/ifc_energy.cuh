@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(32 * NW_, 1)
     pending.kind = kPendNone;
     auto take = [&]() {  // by warp 0, after a block barrier
         if (warp != 0) return;
-        pass_done(L, eq, tot, pending.n0, N, g.tol[eq], true, floor);
+        pass_done(L, eq, tot, pending.n0, N, g.tol[eq], false, true, floor);
         if (tid == 0) last_sq = tot[pending.n0 - 1];
     };
 #pragma unroll 1

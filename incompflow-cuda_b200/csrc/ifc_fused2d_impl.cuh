@@ -329,7 +329,12 @@ int Engine<T>::prepare_persist()
             pa.group = group;
         }
     pa.ks = best_ks;
+    pa.one = persist && persist_grid == pa.tiles.kx * pa.tiles.ky;
     if (!persist) return IFC_OK;
+    pa.npass_m = (n_m + pa.ks - 1) / pa.ks;
+    pa.npass_p = (cfg.n_iter_p + pa.ks - 1) / pa.ks;
+    pa.tail_m = pa.npass_m > 0 ? (pa.npass_m - 1) / pa.group * pa.group : 0;
+    pa.tail_p = pa.npass_p > 0 ? (pa.npass_p - 1) / pa.group * pa.group : 0;
     // SMs that have no tile: narrower tiles, of twelve columns and more, share out
     // the phases between the sweeps (deferred correction, faces, corrections),
     // whose time follows a CTA's own cells; the sweeps cost the same, a region
@@ -351,6 +356,7 @@ int Engine<T>::prepare_persist()
     tg.Ix = w;
     tg.kx = (inner + w - 1) / w;
     persist_grid = tg.kx * tg.ky;
+    pa.one = 1;
     return IFC_OK;
 }
 

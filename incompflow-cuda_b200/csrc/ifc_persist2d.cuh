@@ -157,6 +157,7 @@ constexpr int kMassColumn = 2 * kSetColumns;
 struct LoopState {
     int it, it_begin, it_stop, act, log_level, log_n, status, done;
     int stop[4], sweeps[4];
+    int ends;                   // the pass of the pending decision ends a group
     int hit[4];                 // the early-exit rule was met (it ends the sweeps where a group of passes ends)
     long long cell_updates[4];  // by equation, so that two warps can count at once
     double inner_max_sq[4];     // largest sum of squared changes of a sweep; negative: none yet
@@ -166,8 +167,11 @@ struct LoopState {
 struct PersistArgs {
     int n_iter[4];
     int pin;
-    int ks;          // sweeps per pass
-    int group;       // passes per early-exit check: the sweeps end early after a multiple of ks * group only
+    int one;               // one tile per CTA
+    int ks;                // sweeps per pass
+    int npass_m, npass_p;  // momentum and p' passes
+    int group;             // passes per early-exit check: the sweeps end early after a multiple of ks * group only
+    int tail_m, tail_p;    // the first pass of a phase's last group
     TileGrid tiles;  // tiles for a halo of 2*ks cells
     int stall_test;  // failure-detection test: CTA 0 leaves before its first barrier
 };
@@ -203,9 +207,10 @@ static __device__ __noinline__ int exit_rule(double own, double before, double f
 // us per pass) is only evaluated when some sweep comes within a factor of the
 // tolerance; otherwise the smallest and the largest sum show that none meets
 // it.  Sums are not negative, so they order as their bits do.
-// ends: the pass ends a group, so the sweeps may end here.
+// grouped: several passes per check; ends: the pass ends a group, so the sweeps
+// may end here.
 __device__ __forceinline__ void pass_done(LoopState &L, int e, const double *sq, int ns, int N, double tol,
-                                          bool ends, double floor = -1e20)
+                                          bool grouped, bool ends, double floor = -1e20)
 {
     const int lane = threadIdx.x & 31;
     const double own = sq[lane < ns ? lane : 0], before = L.inner_max_sq[e];
@@ -223,8 +228,7 @@ __device__ __forceinline__ void pass_done(LoopState &L, int e, const double *sq,
         L.inner_max_sq[e] = mx;
         L.sweeps[e] += ns;
         L.cell_updates[e] += (long long)ns * N;
-        if (stop) L.hit[e] = 1;
-        if (ends && L.hit[e]) L.stop[e] = 1;
+        if (stop || (grouped && L.hit[e])) (ends ? L.stop : L.hit)[e] = 1;
     }
 }
 
@@ -326,10 +330,8 @@ enum { kPendNone = 0, kPendMomentum, kPendP, kPendNorms };
 struct Pending {
     int kind, ncol, n0, n1;
     int part;  // offset of the first column in the partials
-    bool ends; // the pass ends a group
-    __device__ __forceinline__ void set(int k, int p, int columns, int a, int b, bool e = true)
+    __device__ __forceinline__ void set(int k, int p, int columns, int a, int b)
     {
-        ends = e;
         kind = k;
         ncol = columns;
         n0 = a;
@@ -370,7 +372,7 @@ __device__ __forceinline__ void pending_totals(const Pending &pd, const double *
 // block barrier; the outcome is in L after the next one.
 template <typename T>
 __device__ __forceinline__ void decide(const Geo<T> &g, LoopState &L, Ctl *ctl, const double *tot,
-                                       const double &mass_sq, const Pending &pd, int ks)
+                                       const double &mass_sq, const Pending &pd, int ks, bool grouped)
 {
     const int warp = threadIdx.x >> 5;
     if (warp > 1) return;
@@ -380,7 +382,7 @@ __device__ __forceinline__ void decide(const Geo<T> &g, LoopState &L, Ctl *ctl, 
     }
     const int e = warp == 1 ? EQ_V : pd.kind == kPendP ? EQ_P : EQ_U;
     const int n = warp == 1 ? pd.n1 : pd.n0;
-    if (n > 0) pass_done(L, e, tot + (warp == 1 ? ks : 0), n, g.N, g.tol[e], pd.ends);
+    if (n > 0) pass_done(L, e, tot + (warp == 1 ? ks : 0), n, g.N, g.tol[e], grouped, !grouped || L.ends);
 }
 
 // Faces whose loads one thread has in flight in the Rhie-Chow phase, and cells
@@ -402,7 +404,7 @@ __global__ void __launch_bounds__(32 * NW_, 1) k_simple2d(const __grid_constant_
     const int G = gridDim.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ntiles = pa.tiles.kx * pa.tiles.ky;
-    const bool one = ntiles <= G;  // one tile per CTA
+    const bool one = pa.one != 0;  // one tile per CTA
     const int ks = pa.ks;
 
     double *sred = reinterpret_cast<double *>(tile_smem<T>() + RT::END);  // per-thread sums of each sweep
@@ -432,11 +434,6 @@ __global__ void __launch_bounds__(32 * NW_, 1) k_simple2d(const __grid_constant_
     clear_guards<RT, T>();
     __syncthreads();
 
-    const int npass_m = (max(pa.n_iter[0], pa.n_iter[1]) + ks - 1) / ks;
-    const int npass_p = (pa.n_iter[3] + ks - 1) / ks;
-    // the first pass of a phase's last group
-    const int tail_m = npass_m > 0 ? (npass_m - 1) / pa.group * pa.group : 0;
-    const int tail_p = npass_p > 0 ? (npass_p - 1) / pa.group * pa.group : 0;
     bool failed = false;
     unsigned int epoch = 0;
     int set = 0;
@@ -448,7 +445,11 @@ __global__ void __launch_bounds__(32 * NW_, 1) k_simple2d(const __grid_constant_
     auto bv = [&](int q) { return field_view(q ? (T *)f.tmp + N : (T *)f.v, N); };
     auto bp = [&](int q) { return field_view(q ? (T *)f.tmp + 2 * (size_t)N : (T *)f.pc, N); };
 
-    const LanePlace<RT> place(tile_box(pa.tiles, blockIdx.x, nx, ny), ny);  // in the CTA's first tile
+    // The lane's place in the CTA's first tile, kept in FP64 only: in FP32 it is
+    // cheaper to find anew in every pass than to hold (4096x2048 2.85 -> 2.73 ms per
+    // outer iteration; FP64 500x190 104 -> 108 us).
+    constexpr bool kKeepPlace = sizeof(T) == 8;
+    const LanePlace<RT> place(tile_box(pa.tiles, blockIdx.x, nx, ny), ny);
     Pending pending;
     pending.kind = kPendNone;
     // Takes a pending decision at once: with several tiles per CTA (a
@@ -457,7 +458,7 @@ __global__ void __launch_bounds__(32 * NW_, 1) k_simple2d(const __grid_constant_
     auto resolve_now = [&]() {
         pending_totals<NW>(pending, partials, G, tot, &tot_mass);
         __syncthreads();
-        decide<T>(g, L, ctl, tot, tot_mass, pending, ks);
+        decide<T>(g, L, ctl, tot, tot_mass, pending, ks, pa.group > 1);
         __syncthreads();
         pending.kind = kPendNone;
     };
@@ -498,19 +499,19 @@ __global__ void __launch_bounds__(32 * NW_, 1) k_simple2d(const __grid_constant_
             Cells<T, R> u, v;
             bool force = false;
 #pragma unroll 1
-            for (int pass = 0; pass < (npass_m > 0 ? npass_m : 1); ++pass) {
+            for (int pass = 0; pass < (pa.npass_m > 0 ? pa.npass_m : 1); ++pass) {
                 const int ns0 = clamp_sweeps(pa.n_iter[0], pass, ks), ns1 = clamp_sweeps(pa.n_iter[1], pass, ks);
                 // what is known of the early exits so far (the last pass's sums
                 // may still be pending; the first pass starts a new iteration)
                 const bool au = ns0 > 0 && (pass == 0 || !L.stop[EQ_U]);
                 const bool av = ns1 > 0 && (pass == 0 || !L.stop[EQ_V]);
                 if (!au && !av && pass > 0) break;
-                const bool sums = pass < tail_m;
+                const bool sums = pass < pa.tail_m;
                 const bool keep = one && pass > 0;
                 bool cu = au, cv = av;  // whether this pass's u, v count
 #pragma unroll 1
                 for (int t = blockIdx.x; t < ntiles; t += G) {
-                    const LanePlace<RT> pl = one ? place : LanePlace<RT>(tile_box(pa.tiles, t, nx, ny), ny);
+                    const LanePlace<RT> pl = kKeepPlace && one ? place : LanePlace<RT>(tile_box(pa.tiles, t, nx, ny), ny);
                     if (keep) {
                         load_cells<RT, T>(u, bu(mcur), pl, nx, ny, true, kOutside<T>);
                         load_cells<RT, T>(v, bv(mcur), pl, nx, ny, true, kOutside<T>);
@@ -524,7 +525,7 @@ __global__ void __launch_bounds__(32 * NW_, 1) k_simple2d(const __grid_constant_
                     publish<RT, T>(v, 1);
                     __syncthreads();
                     if (pending.kind)
-                        decide<T>(g, L, ctl, tot, tot_mass, pending, ks);
+                        decide<T>(g, L, ctl, tot, tot_mass, pending, ks, pa.group > 1);
                     sweeps2<RT, T>(u, v, a, pl, g.relax[EQ_U], g.relax[EQ_V], force, au ? ns0 : 0,
                                    av ? ns1 : 0, ks, sums, t != (int)blockIdx.x, sred);
                     if (pending.kind) {
@@ -555,7 +556,8 @@ __global__ void __launch_bounds__(32 * NW_, 1) k_simple2d(const __grid_constant_
                     }
                     continue;
                 }
-                pending.set(kPendMomentum, set * set_len, 2 * ks, cu ? ns0 : 0, cv ? ns1 : 0, (pass + 1) % pa.group == 0);
+                pending.set(kPendMomentum, set * set_len, 2 * ks, cu ? ns0 : 0, cv ? ns1 : 0);
+                if (tid == 0 && pa.group > 1) L.ends = ((pass + 1) & (pa.group - 1)) == 0;
                 set ^= 1;
                 if (!one) resolve_now();
             }
@@ -650,15 +652,15 @@ __global__ void __launch_bounds__(32 * NW_, 1) k_simple2d(const __grid_constant_
             Cells<T, R> x;
             bool force = false;
 #pragma unroll 1
-            for (int pass = 0; pass < npass_p; ++pass) {
+            for (int pass = 0; pass < pa.npass_p; ++pass) {
                 const int ns = clamp_sweeps(pa.n_iter[3], pass, ks);
                 if (pass > 0 && L.stop[EQ_P]) break;
-                const bool sums = pass < tail_p;
+                const bool sums = pass < pa.tail_p;
                 const bool keep = one && pass > 0;
                 bool stopped = false;
 #pragma unroll 1
                 for (int t = blockIdx.x; t < ntiles; t += G) {
-                    const LanePlace<RT> pl = one ? place : LanePlace<RT>(tile_box(pa.tiles, t, nx, ny), ny);
+                    const LanePlace<RT> pl = kKeepPlace && one ? place : LanePlace<RT>(tile_box(pa.tiles, t, nx, ny), ny);
                     if (pass == 0) zero_cells<RT, T>(x, pl, nx, ny);
                     else load_cells<RT, T>(x, bp(pcur), pl, nx, ny, keep, kOutside<T>);
                     if (pending.kind) pending_totals<NW>(pending, partials, G, tot, &tot_mass);
@@ -666,7 +668,7 @@ __global__ void __launch_bounds__(32 * NW_, 1) k_simple2d(const __grid_constant_
                     publish<RT, T>(x, 0);
                     __syncthreads();
                     if (pending.kind)
-                        decide<T>(g, L, ctl, tot, tot_mass, pending, ks);
+                        decide<T>(g, L, ctl, tot, tot_mass, pending, ks, pa.group > 1);
                     sweeps1<RT, T>(x, a, pl, g.relax[EQ_P], force, ns, ks, sums, t != (int)blockIdx.x, sred);
                     if (pending.kind) {
                         pending.kind = kPendNone;
@@ -683,7 +685,8 @@ __global__ void __launch_bounds__(32 * NW_, 1) k_simple2d(const __grid_constant_
                     if (tid == 0) pass_count(L, EQ_P, ns, N);
                     continue;
                 }
-                pending.set(kPendP, set * set_len, ks, ns, 0, (pass + 1) % pa.group == 0);
+                pending.set(kPendP, set * set_len, ks, ns, 0);
+                if (tid == 0 && pa.group > 1) L.ends = ((pass + 1) & (pa.group - 1)) == 0;
                 set ^= 1;
                 if (!one) resolve_now();
             }
@@ -691,9 +694,13 @@ __global__ void __launch_bounds__(32 * NW_, 1) k_simple2d(const __grid_constant_
         if (failed) break;
 
         const FieldArr<T> pcc = bp(pcur);  // the current p'
-        if (npass_p == 0) {       // no p' sweeps: p' = 0 (src/Solver.cu:193)
-            // no p' pass takes a decision left over from the momentum passes
-            if (pending.kind) resolve_now();
+        if (pa.npass_p == 0) {       // no p' sweeps: p' = 0 (src/Solver.cu:193)
+            // No p' pass takes a decision left over from the momentum passes; nothing
+            // depends on it any more but the counts.
+            if (pending.kind && tid == 0) {
+                pass_count(L, EQ_U, pending.n0, N);
+                pass_count(L, EQ_V, pending.n1, N);
+            }
 #pragma unroll 1
             for (int t = blockIdx.x; t < ntiles; t += G) {
                 const TileBox tl = tile_box(pa.tiles, t, nx, ny);

@@ -13,7 +13,7 @@
 // without another barrier.  The decisions are taken by two warps while the next
 // pass (after the corrections: the first pass of the next outer iteration)
 // already runs; a pass that the decision makes superfluous is not stored.
-// Waiting for them first costs 3 us per pass of the 65 us that an outer
+// Waiting for them first costs 3 us per pass of the 58 us that an outer
 // iteration of the 512x128 channel takes.  Barrier waits are bounded: a CTA
 // that waits longer than kBarrierTimeoutNs sets the error flag, every CTA leaves
 // the loop, and the host reports IFC_TIMEOUT.  The launch is cooperative, so all
@@ -385,8 +385,7 @@ __device__ __forceinline__ void decide(const Geo<T> &g, LoopState &L, Ctl *ctl, 
     if (n > 0) pass_done(L, e, tot + (warp == 1 ? ks : 0), n, g.N, g.tol[e], grouped, !grouped || L.ends);
 }
 
-// Faces whose loads one thread has in flight in the Rhie-Chow phase, and cells
-// in the corrections.
+// Faces whose loads one thread has in flight in the Rhie-Chow phase.
 constexpr int kFaces = 2;
 
 // The persistent kernel of one region shape.  One-tile CTAs keep the links,

@@ -12,12 +12,15 @@
 // that does not depend on the order of the rows' neighbours runs as packed
 // pairs (half the issue slots).  What bounds it is the latency of a half sweep
 // (barrier, exchange row, shuffle, a chain of eleven operations) and then the
-// issue rate: 40 warp instructions for 64 updates, 320 cycles for a 64x32
-// region (450 with the sums of squared changes), against 640 for 850 cells
-// when unknowns sit in shared memory under a generic index map (about 80
-// instructions per 32 updates: masks, addresses, the compiler's division).
-// Outer iteration of the 1024x256 channel 215 -> 112 us, 4096x2048 5.7 -> 3.0
-// ms, 512x128 65.6 -> 60.9 us, 33x31 cavity 105 -> 84 us.
+// issue rate: 40 warp instructions for 64 updates; a half sweep of a 64x32 region
+// takes about 500 cycles for p' and 800 for u and v together (512x128, counted
+// inside the solve), against 640 for one unknown of 850 cells when unknowns sit
+// in shared memory under a generic index map (about 80 instructions per 32
+// updates: masks, addresses, the compiler's division).  The half sweeps are a
+// third of an outer iteration; the rest is the grid barriers, the turn-round of
+// a pass (halos, links, own cells and column sums) and the faces and corrections.
+// Outer iteration of the 1024x256 channel 215 -> 103 us, 4096x2048 5.7 -> 2.7
+// ms, 512x128 65.6 -> 58 us, 33x31 cavity 105 -> 84 us.
 //
 // The divisor of a point update, the equation's diagonal, does not change
 // within a solve, so z = 1/aC is computed once (IEEE division) and a quotient
@@ -263,7 +266,9 @@ __host__ __device__ inline bool split_axis(int n, int C, int H, int *k, int *I)
 // memory (addressed by 32-bit offsets from there: pointers would cost the
 // sweeps two registers each):
 //   sources of two unknowns: thread-private pairs, [colour][row pair][thread]
-//     (in registers they would push the sweeps over the register limit);
+//     (in registers they would spill more of the sweeps: as it is, regions of 32
+//     rows spill 34 values per thread, of 64 rows 183, FP64 77 to 144, and one
+//     instruction in 80 is a spill at 512x128);
 //   exchange rows of two unknowns: side 0 the warps' first rows, side 1 their
 //     last, a row of zeros at either end, columns split by parity.
 template <typename T, int R_, int NW_>
